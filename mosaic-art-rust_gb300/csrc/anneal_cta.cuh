@@ -1,328 +1,521 @@
-// anneal_cta.cuh -- one simulated-annealing chain by one CTA of kChainWarps
-// warps (anneal_cta_kernel, for single mosaics and for every chain of a batch;
-// the one-warp chain of anneal_chain.cuh, whose rules this follows exactly, is
-// the fallback when the CTA form does not fit in shared memory).
+// anneal_cta.cuh -- one simulated-annealing chain by one CTA (anneal_cta_kernel,
+// for single mosaics and for every chain of a batch).
 //
 // Reference: optimizer.rs:41-129 MosaicOptimizer::optimize, optimizer.rs:132-198
 // optimize_greedy, adjacency.rs:133-214 calculate_swap_delta.
 //
-// A chain is a sequence of dependent swaps, and a single proposal is a long
-// dependent chain of instructions, so a round evaluates kRound consecutive
-// proposals at once (eight lanes each, as in anneal_chain.cuh) on the same grid
-// and commits them in order, up to the first proposal that reads a cell within
-// Manhattan distance 1 of an earlier accepted swap of the round; the next round
-// re-evaluates that one on the updated grid.  Per round:
-//  1. every group evaluates its proposal: skip flag, delta (the reference's
-//     summation order), and publishes them with its positions;
-//  2. after one barrier every warp derives the same round outcome redundantly:
-//     lanes 0..kRound-1 take one proposal each -- its temperature (the chain's T
-//     times the decay once per earlier non-skipped proposal of the round,
-//     multiplied step by step), its acceptance (this library's exp), then the
-//     earlier-accepted-neighbour test over all pairs (lanes split the pairs,
-//     one OR reduction) -- and every thread runs the in-order commit
-//     bookkeeping (running cost, best, counters, temperature);
-//  3. the groups of committed accepted proposals swap their two cells; a
-//     second barrier ends the round.
-// Whether a proposal is skipped does not depend on the grid (swaps never move
-// empty cells), so step 2 needs nothing from the commit itself.  Random
-// numbers: the same counter-based Philox stream as anneal_chain.cuh (a CPU
-// replay of the stream makes the same decisions); every thread of the CTA
-// decodes one proposal per refill of a shared ring.
+// A chain is a sequence of dependent swaps, so its speed is the latency from
+// one swap to the next that reads its cells.  Almost everything about a
+// proposal is known ahead of the chain: its two cells (a counter-based draw),
+// whether it is skipped (swaps never move empty cells, so emptiness is a
+// property of the start grid), its temperature (the decay is applied once per
+// earlier proposal that is not skipped, whatever was accepted) and with it the
+// deltas that are accepted; and which earlier proposals can matter to it: those
+// that may swap a cell it reads, i.e. with a position within Manhattan distance
+// 1 of its own.  Only the eight neighbour weights need the grid.  So the work is
+// split by warp, window of 64 proposals by window:
+//   * kProducers warps take a window each in turn: draw and decode, skip flags,
+//     the window's temperatures (one chain of multiplications, handed from
+//     window to window), the acceptance bounds, and each proposal's level --
+//     0 when no earlier proposal of the window is near it, else one more than
+//     the highest level among those that are;
+//   * kEvalWarps warps evaluate a window level by level, four lanes a proposal
+//     (one direction each: a neighbour of either position), decide and swap.
+//     Proposals of one level do not
+//     touch one another's cells, and a proposal comes after every earlier one
+//     near it, so each reads the grid exactly as the sequential chain would;
+//   * one warp keeps the books two windows behind: the running cost is summed in
+//     proposal order, with the best cost and the counters.
+// Acceptance: u < exp(-delta / T) is decided by comparing delta with -T ln u
+// when it lies further from it than 1e-4 T (over ten times the error of the
+// logarithm, the division and this library's exp together), else by the
+// definition itself.
+// The warps meet at named barriers only (no spinning): FULL[slot] when a window
+// is prepared and the one two before it is done (producer, evaluators, book
+// keeper), EMPTY[slot] when the evaluators hold a window's descriptors in
+// registers, TEMP[slot] when a window's first temperature is known, EVAL between
+// levels and windows.
+//
+// What bounds it: the latency of a level (shared-memory reads of cells, then
+// Lab; square roots and reciprocals; the in-order sum of eight terms; a
+// barrier).  A window of 64 takes ~2 000 cycles on a 24 000-cell grid (1.9
+// levels on average), issue slots 39% used.  Before, a CTA of four warps drew,
+// evaluated, tested all pairs for conflicts and booked 32 (or 16) proposals in
+// turn, ~4 000 (2 550) cycles a round.  Measured, GB300, before -> now:
+// 64 chains x 100 000 iterations on 179 x 134 cells 6.32 -> 1.53 ms; 32 x 2000
+// on 80 x 60 0.203 -> 0.058 ms.  Windows of 32, eight lanes a proposal (16
+// warps), and two proposals a group of eight lanes were measured too: 2.1, 1.55
+// and 2.0 ms on the first.
 #pragma once
-#include "anneal_chain.cuh"
+#include "mg_internal.h"
+#include "roots.cuh"
 
 namespace mg {
-namespace anneal_cta_detail {
-using anneal_detail::kNone16;
-using anneal_detail::wgt;
+namespace anneal_detail {
 
-constexpr int kChainWarps = 4;
-constexpr int kThreads = kChainWarps * 32;
-// Proposals per round: 16 (eight lanes each, one neighbour term a lane) or,
-// on large grids, where two proposals of a round rarely touch, 32 (four lanes
-// each, two terms a lane): about as long a round, nearly twice the swaps.
-constexpr int kRoundMax = 32;
-constexpr int kCtaRing = 4 * kThreads;   // decoded proposals in shared memory
+constexpr uint16_t kNone16 = 0xFFFFu;  // a cell without a tile
+constexpr int kWindow = 64;     // proposals per window
+constexpr int kEvalWarps = 8;   // four lanes a proposal
+constexpr int kEval = kEvalWarps * 32;
+constexpr int kProducers = 4;   // warps preparing windows, two proposals a lane; also the descriptor slots
+constexpr int kThreads = kEval + 32 * kProducers + 32;
+// named barriers (0 is __syncthreads)
+constexpr int kBarFull = 1, kBarEmpty = kBarFull + kProducers, kBarTemp = kBarEmpty + kProducers,
+              kBarEval = kBarTemp + kProducers;
+static_assert(kBarEval < 16, "sixteen barriers a CTA");
 
-struct RoundSlot {  // one proposal's outcome of step 1
-  float delta;
-  float u;              // acceptance uniform
-  uint32_t flags;       // bit 0: skipped
-  uint32_t pos1, pos2;  // x | y << 16
-  uint32_t pad[3];
+struct Proposal {        // a prepared proposal
+  int p1, p2;            // cells
+  uint32_t flags;        // bits 0-7: neighbour t lies in the grid and is not the other position; 8: adjacent
+                         // positions; 9-10: direction of pos2 from pos1; 11: not skipped; 16-21: level
+  float lo;              // accepted when delta < lo (delta < 0 always is)
+  float hi;              // rejected when delta > hi
+  float u, t;            // acceptance uniform, temperature
+  int levels;            // levels of the window
+};
+struct Outcome {  // a window's decisions, for the book keeper
+  float delta[kWindow];     // 0 unless accepted
+  uint32_t flags[kWindow];  // bit 0: accepted, 1: not skipped
+};
+constexpr int kTermStride = 36;  // floats between the sets of a warp's terms (four banks apart)
+struct ChainShared {
+  Proposal ring[kProducers][kWindow];
+  Outcome out[3];
+  float terms[kEvalWarps][4 * kTermStride];  // old, old, new, new weights: neighbours of pos1, of pos2
+  int2 pos[kProducers][kWindow];           // a window's positions, as near_pos takes them
+  float temps[kProducers][kWindow + 4];    // the window's first temperature after 0, 1, ... coolings
+  float temp[kProducers];                  // first temperature of the window in the slot
+  float sums[kWindow];                     // the running cost after each proposal of a window
 };
 
-__host__ __device__ inline size_t anneal_cta_smem_bytes(int max_cells, int p, bool lab_smem) {
-  return (size_t)kCtaRing * 16 + (size_t)kRoundMax * sizeof(RoundSlot) + (lab_smem ? (size_t)p * 16 : 0) +
-         (((size_t)max_cells * 2 + 15) & ~(size_t)15);
+// Behind it: the writers table (kProducers x 2 x writer_slots words), the
+// palette Lab, the grid (one 16-bit material a cell, and an empty cell n).
+// More table slots leave fewer chance hits; the largest grids leave room for few.
+constexpr int kWriterSlots = 4096, kWriterSlotsShared = 512, kWriterSlotsMin = 64;
+__host__ __device__ inline size_t anneal_cta_smem_bytes(int max_cells, int p, bool lab_smem, int writer_slots) {
+  return sizeof(ChainShared) + (size_t)kProducers * 2 * 4 * writer_slots + (lab_smem ? (size_t)p * 16 : 0) +
+         ((((size_t)max_cells + 1) * 2 + 15) & ~(size_t)15);
+}
+static_assert(sizeof(ChainShared) % 16 == 0, "16-byte aligned parts");
+
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+constexpr int kFullThreads = 32 + kEval + 32, kEmptyThreads = kEval + 32, kTempThreads = 64;
+
+// Positions y * S + x with S >= gw + 2: within Manhattan distance 1 exactly
+// when they differ by 0, 1 or S.
+__device__ __forceinline__ bool near_pos(int a, int b, int S) {
+  const int d = abs(a - b);
+  return d <= 1 || d == S;
 }
 
-template <bool kLabSmem, int kRound>
+// Producer `slot`: prepares windows slot, slot + kProducers, ...; a lane holds
+// proposals lane and lane + 32 (h = 0, 1).
+__device__ __forceinline__ void produce_windows(const AnnealJob& J, int chain, long long windows, int slot,
+                                                ChainShared& S, uint32_t* writers, int writer_slots,
+                                                const uint16_t* s_grid) {
+  const int lane = threadIdx.x & 31;
+  const int gw = J.gw, gh = J.gh, stride = gw + 2;
+  const bool greedy_only = J.greedy_only != 0;
+  const float decay = J.decay, inf = __int_as_float(0x7f800000);
+  const unsigned below = (1u << lane) - 1u;
+  int2* pos = S.pos[slot];
+  float* temps = S.temps[slot];
+  uint2* table = reinterpret_cast<uint2*>(writers) + (size_t)slot * writer_slots;
+  const unsigned tmask = (unsigned)writer_slots - 1u;
+  for (long long w = slot; w < windows; w += kProducers) {
+    int x1[2], y1[2], x2[2], y2[2], c1[2], c2[2];
+    float u[2];
+    bool skip[2];
+    unsigned live[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long my = w * kWindow + 32 * h + lane;
+      const uint32_t hi32 = (uint32_t)((unsigned long long)my >> 32);
+      const u32x4 a = philox((uint32_t)my, (uint32_t)chain, J.stream, 2u * hi32, J.key0, J.key1);
+      const u32x4 b = philox((uint32_t)my, (uint32_t)chain, J.stream, 2u * hi32 + 1u, J.key0, J.key1);
+      x1[h] = (int)range_u32(a.x, (uint32_t)gw);
+      y1[h] = (int)range_u32(a.y, (uint32_t)gh);
+      x2[h] = (int)range_u32(a.z, (uint32_t)gw);
+      y2[h] = (int)range_u32(a.w, (uint32_t)gh);
+      u[h] = unit_f32(b.x);
+      c1[h] = y1[h] * gw + x1[h];
+      c2[h] = y2[h] * gw + x2[h];
+      // emptiness never changes, so reading beside the evaluators' swaps is safe
+      skip[h] = my >= J.iters || c1[h] == c2[h] || s_grid[c1[h]] == kNone16 || s_grid[c2[h]] == kNone16;
+      live[h] = __ballot_sync(0xffffffffu, !skip[h]);
+      pos[32 * h + lane] = make_int2(y1[h] * stride + x1[h], y2[h] * stride + x2[h]);
+    }
+
+    // ---- temperatures: the window's first one comes from the window before.
+    // One chain of multiplications; each lane then picks its own.
+    if (!greedy_only) {
+      if (w > 0) bar_sync(kBarTemp + slot, kTempThreads);
+      float tk = w > 0 ? S.temp[slot] : J.t0;
+#pragma unroll
+      for (int k = 0; k < kWindow; k += 4) {
+        float4 v;
+        v.x = tk;
+        v.y = __fmul_rn(v.x, decay);
+        v.z = __fmul_rn(v.y, decay);
+        v.w = __fmul_rn(v.z, decay);
+        tk = __fmul_rn(v.w, decay);
+        *reinterpret_cast<float4*>(temps + k) = v;
+      }
+      temps[kWindow] = tk;
+      __syncwarp();
+      if (w + 1 < windows) {
+        const int next = (slot + 1) % kProducers;
+        if (lane == 0) S.temp[next] = temps[__popc(live[0]) + __popc(live[1])];
+        __syncwarp();
+        bar_arrive(kBarTemp + next, kTempThreads);
+      }
+    }
+
+    // ---- levels.  The writers table holds, per (hashed) cell, which proposals
+    // of the window may swap it; a proposal looks up the ten cells it reads,
+    // keeps the earlier ones and checks each against the positions (chance hits
+    // of the hash drop out).
+    auto at = [&](int c) -> uint2& { return table[(unsigned)c & tmask]; };
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (!skip[h]) {
+        uint32_t* t1 = h ? &at(c1[h]).y : &at(c1[h]).x;
+        uint32_t* t2 = h ? &at(c2[h]).y : &at(c2[h]).x;
+        atomicOr(t1, 1u << lane);
+        atomicOr(t2, 1u << lane);
+      }
+    __syncwarp();
+    unsigned e0 = 0u, e10 = 0u, e11 = 0u;  // earlier proposals near this lane's: h = 0's; h = 1's in either half
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int a = e ? c2[0] : c1[0], b = e ? c2[1] : c1[1];
+      e0 |= at(a).x | at(a - 1).x | at(a + 1).x | at(a - gw).x | at(a + gw).x;
+      const int bs[5] = {b, b - 1, b + 1, b - gw, b + gw};
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const uint2 v = at(bs[k]);
+        e10 |= v.x;
+        e11 |= v.y;
+      }
+    }
+    e0 = skip[0] ? 0u : e0 & below;
+    e10 = skip[1] ? 0u : e10;
+    e11 = skip[1] ? 0u : e11 & below;
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (!skip[h]) at(c1[h]) = at(c2[h]) = make_uint2(0u, 0u);
+    {
+      const int2 q0 = pos[lane], q1 = pos[32 + lane];
+      unsigned m0 = e0, m10 = e10, m11 = e11;
+      while (__any_sync(0xffffffffu, (m0 | m10 | m11) != 0u)) {
+        // the next unchecked one of the lane: h = 0's first
+        const bool f0 = m0 != 0u, f1 = !f0 && m10 != 0u;
+        const unsigned m = f0 ? m0 : (f1 ? m10 : m11);
+        const int k = (__ffs(m) - 1) & 31;
+        const int2 f = pos[k + ((f0 || f1) ? 0 : 32)];
+        const int a = f0 ? q0.x : q1.x, b = f0 ? q0.y : q1.y;
+        const bool close = near_pos(f.x, a, stride) || near_pos(f.x, b, stride) || near_pos(f.y, a, stride) ||
+                           near_pos(f.y, b, stride);
+        const unsigned bit = m & (0u - m), drop = close ? 0u : bit;
+        m0 &= f0 ? ~bit : ~0u;
+        e0 &= f0 ? ~drop : ~0u;
+        m10 &= f1 ? ~bit : ~0u;
+        e10 &= f1 ? ~drop : ~0u;
+        m11 &= (f0 || f1) ? ~0u : ~bit;
+        e11 &= (f0 || f1) ? ~0u : ~drop;
+      }
+    }
+    int level[2] = {0, 0}, levels = 1;
+    unsigned done0 = __ballot_sync(0xffffffffu, e0 == 0u), done1 = __ballot_sync(0xffffffffu, (e10 | e11) == 0u);
+    for (; (done0 & done1) != 0xffffffffu; ++levels) {
+      const bool now0 = !((done0 >> lane) & 1u) && (e0 & ~done0) == 0u;
+      const bool now1 = !((done1 >> lane) & 1u) && ((e10 & ~done0) | (e11 & ~done1)) == 0u;
+      level[0] = now0 ? levels : level[0];
+      level[1] = now1 ? levels : level[1];
+      done0 |= __ballot_sync(0xffffffffu, now0);
+      done1 |= __ballot_sync(0xffffffffu, now1);
+    }
+    __syncwarp();
+
+    // the slot is free once the evaluators hold the window kProducers back
+    if (w >= kProducers) bar_sync(kBarEmpty + slot, kEmptyThreads);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      // the acceptance bounds
+      float lo = 0.0f, hi = 0.0f, t = 0.0f;
+      if (!greedy_only) {
+        t = temps[__popc(live[h] & below) + (h ? __popc(live[0]) : 0)];
+        const bool ok = u[h] > 0.0f && t >= 1e-30f && t <= 1e30f;
+        const float theta = -t * __logf(u[h]), margin = 1e-4f * t;
+        lo = ok ? fmaxf(theta - margin, 0.0f) : -inf;
+        hi = ok ? theta + margin : inf;
+      }
+      const int dx = x2[h] - x1[h], dy = y2[h] - y1[h];
+      const bool adjacent = (dx == 0 && (dy == 1 || dy == -1)) || (dy == 0 && (dx == 1 || dx == -1));
+      const uint32_t dir12 = dy == -1 ? 0u : (dy == 1 ? 1u : (dx == -1 ? 2u : 3u));
+      uint32_t flags = (y1[h] > 0 ? 1u : 0u) | (y1[h] < gh - 1 ? 2u : 0u) | (x1[h] > 0 ? 4u : 0u) |
+                       (x1[h] < gw - 1 ? 8u : 0u) | (y2[h] > 0 ? 16u : 0u) | (y2[h] < gh - 1 ? 32u : 0u) |
+                       (x2[h] > 0 ? 64u : 0u) | (x2[h] < gw - 1 ? 128u : 0u);
+      flags = adjacent ? (flags & ~((1u << dir12) | (16u << (dir12 ^ 1u)))) | 0x100u | (dir12 << 9) : flags;
+      flags |= (skip[h] ? 0u : 0x800u) | ((uint32_t)level[h] << 16);
+      int4* d = reinterpret_cast<int4*>(&S.ring[slot][32 * h + lane]);
+      d[0] = make_int4(c1[h], c2[h], (int)flags, __float_as_int(lo));
+      d[1] = make_int4(__float_as_int(hi), __float_as_int(u[h]), __float_as_int(t), levels);
+    }
+    __syncwarp();
+    bar_arrive(kBarFull + slot, kFullThreads);
+  }
+}
+
+// The evaluators: the group of four lanes g of warp v takes proposal 8 v + g of
+// a window, lane `dir` the neighbour of each position in one direction (up,
+// down, left, right).
+template <bool kLabSmem>
+__device__ __forceinline__ void evaluate_windows(const float4* __restrict__ pal, int p, const AnnealJob& J,
+                                                 long long windows, ChainShared& S, const float4* s_lab,
+                                                 uint16_t* s_grid) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gw = J.gw, n = gw * J.gh;
+  const bool greedy_only = J.greedy_only != 0;
+  const int grp = lane >> 2, dir = lane & 3;
+  const int q = warp * 8 + grp;
+  const int step = dir == 0 ? -gw : (dir == 1 ? gw : (dir == 2 ? -1 : 1));
+  float* put = &S.terms[warp][lane];
+  // even lanes sum the old weights, odd lanes the new ones
+  const float* get = &S.terms[warp][(dir & 1) * 2 * kTermStride + grp * 4];
+  const uint32_t last = (uint32_t)max(p - 1, 0);
+  auto lab = [&](uint16_t g) -> float4 {  // a colour of the palette for an empty cell, too
+    const uint32_t i = min((uint32_t)g, last);
+    return kLabSmem ? s_lab[i] : __ldg(pal + i);
+  };
+  // A window's descriptor, read while the window before it waits for its cells.
+  struct Desc {
+    int p1, p2, n1, n2, level, levels;
+    uint32_t flags;
+    float lo, hi, u, t;
+  };
+  int slot = 0;
+  auto take = [&](long long w) -> Desc {
+    bar_sync(kBarFull + slot, kFullThreads);
+    const int4 d = *reinterpret_cast<const int4*>(&S.ring[slot][q]);
+    const int4 e = *(reinterpret_cast<const int4*>(&S.ring[slot][q]) + 1);
+    Desc D;
+    D.p1 = d.x;
+    D.p2 = d.y;
+    D.flags = (uint32_t)d.z;
+    D.lo = __int_as_float(d.w);
+    D.hi = __int_as_float(e.x);
+    D.u = __int_as_float(e.y);
+    D.t = __int_as_float(e.z);
+    D.levels = e.w;
+    D.level = (D.flags & 0x800u) ? (int)((D.flags >> 16) & 63u) : -1;
+    const bool mutual = (D.flags & 0x100u) != 0u && dir == (int)((D.flags >> 9) & 3u);
+    // cell n of the grid is an empty one for the neighbours outside it
+    D.n1 = (((D.flags >> dir) & 1u) || mutual) ? D.p1 + step : n;
+    D.n2 = ((D.flags >> (4 + dir)) & 1u) ? D.p2 + step : n;
+    if (w + kProducers < windows) bar_arrive(kBarEmpty + slot, kEmptyThreads);
+    slot = slot + 1 == kProducers ? 0 : slot + 1;
+    return D;
+  };
+  // Proposal D, whose cells hold g1 and g2, this lane's neighbours a1 and a2.
+  auto decide = [&](const Desc& D, uint16_t g1, uint16_t g2, uint16_t a1, uint16_t a2, Outcome& O, bool act) {
+    const float4 l1 = lab(g1), l2 = lab(g2), c1 = lab(a1), c2 = lab(a2);
+    const float2 u1 = weight_of_sq2(sq_dist(l1.x, l1.y, l1.z, c1.x, c1.y, c1.z),
+                                    sq_dist(l2.x, l2.y, l2.z, c1.x, c1.y, c1.z));
+    const float2 u2 = weight_of_sq2(sq_dist(l1.x, l1.y, l1.z, c2.x, c2.y, c2.z),
+                                    sq_dist(l2.x, l2.y, l2.z, c2.x, c2.y, c2.z));
+    const bool use1 = ((D.flags >> dir) & 1u) && a1 != kNone16, use2 = a2 != kNone16;
+    put[0] = use1 ? u1.x : 0.0f;
+    put[kTermStride] = use2 ? u2.y : 0.0f;
+    put[2 * kTermStride] = use1 ? u1.y : 0.0f;
+    put[3 * kTermStride] = use2 ? u2.x : 0.0f;
+    __syncwarp();
+    // the reference's order of summation
+    const float4 s0 = *reinterpret_cast<const float4*>(get), s1 = *reinterpret_cast<const float4*>(get + kTermStride);
+    float cost = __fadd_rn(__fadd_rn(s0.x, s0.y), s0.z);  // weights are >= 0: 0 + s0.x is s0.x
+    cost = __fadd_rn(__fadd_rn(cost, s0.w), s1.x);
+    cost = __fadd_rn(__fadd_rn(cost, s1.y), s1.z);
+    cost = __fadd_rn(cost, s1.w);
+    if (__any_sync(0xffffffffu, (D.flags & 0x100u) != 0u)) {  // the mutual weight, last on both sides
+      const float m = __shfl_sync(0xffffffffu, u1.x, (grp << 2) + (int)((D.flags >> 9) & 3u));
+      if (D.flags & 0x100u) cost = __fadd_rn(cost, m);
+    }
+    const float other = __shfl_xor_sync(0xffffffffu, cost, 1);
+    if (dir == 0 && act) {
+      const float delta = g1 == g2 ? 0.0f : __fsub_rn(other, cost);
+      bool accept = delta < D.lo;
+      if (!accept && !(delta > D.hi))
+        accept = delta < 0.0f || (!greedy_only && D.u < exp_spec(__fdiv_rn(-delta, D.t)));
+      if (accept) {
+        s_grid[D.p1] = g2;
+        s_grid[D.p2] = g1;
+      }
+      O.delta[q] = accept ? delta : 0.0f;
+      O.flags[q] = accept ? 3u : 2u;
+    }
+    __syncwarp();  // the terms are read before the next level writes them
+  };
+  Desc next{};
+  if (windows > 0) next = take(0);
+  int o = 0;  // the window's outcome slot
+  for (long long w = 0; w < windows; ++w) {
+    const Desc D = next;
+    Outcome& O = S.out[o];
+    o = o == 2 ? 0 : o + 1;
+    {
+      const uint16_t g1 = s_grid[D.p1], g2 = s_grid[D.p2], a1 = s_grid[D.n1], a2 = s_grid[D.n2];
+      if (w + 1 < windows) next = take(w + 1);
+      if (__any_sync(0xffffffffu, D.level == 0)) decide(D, g1, g2, a1, a2, O, D.level == 0);
+      if (D.level < 0 && dir == 0) {
+        O.delta[q] = 0.0f;
+        O.flags[q] = 0u;
+      }
+    }
+    for (int l = 1; l < D.levels; ++l) {
+      bar_sync(kBarEval, kEval);
+      if (__any_sync(0xffffffffu, D.level == l))
+        decide(D, s_grid[D.p1], s_grid[D.p2], s_grid[D.n1], s_grid[D.n2], O, D.level == l);
+    }
+    __syncwarp();
+    bar_sync(kBarEval, kEval);  // the window's swaps are in place
+  }
+}
+
+// One chain by one CTA of kThreads threads.  smem: anneal_cta_smem_bytes bytes, 16-byte
+// aligned; writer_slots a power of two.
+template <bool kLabSmem>
 __device__ __forceinline__ void anneal_chain_cta(const float4* __restrict__ pal, int p, const AnnealJob& J, int chain,
-                                                 uint8_t* smem) {
-  static_assert(kRound == 16 || kRound == 32, "16 or 32 proposals a round");
-  constexpr int kL = kThreads / kRound;  // lanes per proposal: 8 or 4
-  constexpr int kT = 8 / kL;             // neighbour terms per lane: 1 or 2
-  constexpr int kConfPerWarp = (kRound - 1 + kChainWarps - 1) / kChainWarps;  // conflict tests per warp
+                                                 int writer_slots, uint8_t* smem) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gw = J.gw, gh = J.gh, n = gw * gh;
-  __shared__ unsigned s_conf[kChainWarps];  // written after the round's first barrier, read after the second
-  int4* s_ring = reinterpret_cast<int4*>(smem);
-  RoundSlot* s_round = reinterpret_cast<RoundSlot*>(smem + (size_t)kCtaRing * 16);
-  float4* s_lab = reinterpret_cast<float4*>(smem + (size_t)kCtaRing * 16 + (size_t)kRoundMax * sizeof(RoundSlot));
-  uint16_t* s_grid = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(s_lab) +
-                                                 (kLabSmem ? (size_t)p * sizeof(float4) : 0));
+  ChainShared& S = *reinterpret_cast<ChainShared*>(smem);
+  uint32_t* writers = reinterpret_cast<uint32_t*>(smem + sizeof(ChainShared));
+  float4* s_lab = reinterpret_cast<float4*>(writers + kProducers * 2 * writer_slots);
+  uint16_t* s_grid = reinterpret_cast<uint16_t*>(s_lab + (kLabSmem ? p : 0));
   if (kLabSmem)
     for (int i = tid; i < p; i += kThreads) s_lab[i] = pal[i];
-  for (int i = tid; i < n; i += kThreads) {
-    const int g = __ldcg(J.grid_in + i);
+  for (int i = tid; i <= n; i += kThreads) {
+    const int g = i < n ? __ldcg(J.grid_in + i) : -1;
     s_grid[i] = g < 0 ? kNone16 : (uint16_t)g;
   }
+  for (int i = tid; i < kProducers * 2 * writer_slots; i += kThreads) writers[i] = 0u;
   __syncthreads();
-  auto lab = [&](int i) -> float4 { return kLabSmem ? s_lab[i] : __ldg(pal + i); };
+  const long long windows = (J.iters + kWindow - 1) / kWindow;
 
-  // Initial cost: calculate_total_cost of the start grid (sequential FP32 sum).
-  float current;
-  if (J.initial_cost) {
-    current = __ldcg(J.initial_cost);
+  if (warp < kEvalWarps) {
+    evaluate_windows<kLabSmem>(pal, p, J, windows, S, s_lab, s_grid);
+    __syncthreads();
+  } else if (warp < kEvalWarps + kProducers) {
+    produce_windows(J, chain, windows, warp - kEvalWarps, S, writers, writer_slots, s_grid);
+    __syncthreads();
   } else {
-    current = 0.0f;
-    for (int c0 = 0; c0 < n; c0 += 32) {
-      const int c = c0 + lane;
-      float tr = 0.0f, td = 0.0f;
-      if (c < n) {
-        const int x = c % gw, y = c / gw;
-        const uint16_t cur = s_grid[c];
-        if (cur != kNone16) {
-          const float4 lc = lab(cur);
-          if (x < gw - 1 && s_grid[c + 1] != kNone16) tr = wgt(lc, lab(s_grid[c + 1]));
-          if (y < gh - 1 && s_grid[c + gw] != kNone16) td = wgt(lc, lab(s_grid[c + gw]));
+    // ---- the book keeper.  Initial cost: calculate_total_cost of the start
+    // grid (sequential FP32 sum), read from global memory as the evaluators may
+    // be swapping already.
+    float current;
+    if (J.initial_cost) {
+      current = __ldcg(J.initial_cost);
+    } else {
+      auto lab = [&](int i) -> float4 { return kLabSmem ? s_lab[i] : __ldg(pal + i); };
+      current = 0.0f;
+      for (int c0 = 0; c0 < n; c0 += 32) {
+        const int c = c0 + lane;
+        float tr = 0.0f, td = 0.0f;
+        if (c < n) {
+          const int x = c % gw, y = c / gw;
+          const int cur = __ldcg(J.grid_in + c);
+          if (cur >= 0) {
+            const float4 lc = lab(cur);
+            const int r = x < gw - 1 ? __ldcg(J.grid_in + c + 1) : -1, d = y < gh - 1 ? __ldcg(J.grid_in + c + gw) : -1;
+            if (r >= 0) tr = wgt(lc, lab(r));
+            if (d >= 0) td = wgt(lc, lab(d));
+          }
+        }
+        const int cnt = min(32, n - c0);
+        for (int s = 0; s < cnt; ++s) {
+          current = __fadd_rn(current, __shfl_sync(0xffffffffu, tr, s));
+          current = __fadd_rn(current, __shfl_sync(0xffffffffu, td, s));
         }
       }
-      const int cnt = min(32, n - c0);
-      for (int s = 0; s < cnt; ++s) {
-        current = __fadd_rn(current, __shfl_sync(0xffffffffu, tr, s));
-        current = __fadd_rn(current, __shfl_sync(0xffffffffu, td, s));
-      }
     }
-  }
-  const float initial = current;
-  float best = current;
-  long long accepted = 0, improved = 0, cooled = 0;
-  float temp = J.t0;
-  const float decay = J.decay;
-  const bool greedy_only = J.greedy_only != 0;
-  const uint32_t k0 = J.key0, k1 = J.key1, strm = J.stream;
-  const long long iters = J.iters;
-  const int grp = lane / kL, slot = lane % kL, leader = grp * kL;
-  const int q_mine = warp * (32 / kL) + grp;  // this group's proposal within the round
-
-  long long it = 0, filled = 0;
-  while (it < iters) {
-    // ---- refill the ring (uniform condition) ---------------------------------------
-    if (filled < iters && filled - it < kRound) {
-      const long long my = filled + tid;
-      if (my < iters) {
-        const uint32_t hi = (uint32_t)((unsigned long long)my >> 32);
-        const u32x4 a = philox((uint32_t)my, (uint32_t)chain, strm, 2u * hi, k0, k1);
-        const u32x4 b = philox((uint32_t)my, (uint32_t)chain, strm, 2u * hi + 1u, k0, k1);
-        const uint32_t x1 = range_u32(a.x, (uint32_t)gw), y1 = range_u32(a.y, (uint32_t)gh);
-        const uint32_t x2 = range_u32(a.z, (uint32_t)gw), y2 = range_u32(a.w, (uint32_t)gh);
-        s_ring[my & (kCtaRing - 1)] = make_int4((int)(x1 | (y1 << 16)), (int)(x2 | (y2 << 16)),
-                                                __float_as_int(unit_f32(b.x)), 0);
-      }
-      filled += kThreads;
-      __syncthreads();
-    }
-    // ---- 1. evaluate proposal it + q_mine ------------------------------------------------
-    // Branch-free: every lane of a group computes two weights on clamped
-    // operands and keeps what its slot needs (lanes 0-3: neighbours of pos1 in
-    // up, down, left, right order; 4-7: those of pos2).
-    const long long i = it + q_mine;
-    const bool live = i < iters;
-    const int4 e = s_ring[(live ? i : it) & (kCtaRing - 1)];
-    const int x1 = e.x & 0xFFFF, y1 = (e.x >> 16) & 0xFFFF, x2 = e.y & 0xFFFF, y2 = (e.y >> 16) & 0xFFFF;
-    const int p1 = y1 * gw + x1, p2 = y2 * gw + x2;
-    const uint16_t g1 = s_grid[p1], g2 = s_grid[p2];
-    const bool skip = !live || p1 == p2 || g1 == kNone16 || g2 == kNone16;
-    const bool same = g1 == g2;
-    float old_cost = 0.0f, new_cost = 0.0f, m0 = 0.0f;
-    if constexpr (kT == 1) {
-      const bool first = slot < 4;
-      const int dir = slot & 3;
-      const int bx = first ? x1 : x2, by = first ? y1 : y2;
-      const int nx = bx + (dir == 2 ? -1 : (dir == 3 ? 1 : 0)), ny = by + (dir == 0 ? -1 : (dir == 1 ? 1 : 0));
-      const bool inb = nx >= 0 && nx < gw && ny >= 0 && ny < gh;
-      const int nb = inb ? ny * gw + nx : p1;
-      const bool mutual = inb && nb == (first ? p2 : p1);
-      const uint16_t an = s_grid[nb];
-      const bool work = !skip && !same && inb;
-      const bool nbr = work && !mutual && an != kNone16;  // a placed neighbour
-      const uint16_t gs1 = skip ? (uint16_t)0 : g1, gs2 = skip ? (uint16_t)0 : g2;
-      const uint16_t c_idx = mutual ? gs2 : (an != kNone16 ? an : gs1);
-      const float4 la1 = lab(gs1), la2 = lab(gs2), lc = lab(c_idx);
-      const float w1 = wgt(la1, lc), w2 = wgt(la2, lc);
-      const float o = nbr ? (first ? w1 : w2) : 0.0f;
-      const float nw = nbr ? (first ? w2 : w1) : 0.0f;
-      m0 = (work && mutual && first) ? w1 : 0.0f;
+    const float initial = current;
+    float best = current;
+    long long accepted = 0, cooled = 0, improved = 0;
+    // A proposal that was not accepted adds 0 and is no new best, so every
+    // proposal is booked alike: one chain of additions, its partial sums to
+    // shared memory; when one of them is a new best, each lane compares two of
+    // them with the least before.
+    auto book = [&](const Outcome& O) {
+      float d[kWindow];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        old_cost = __fadd_rn(old_cost, __shfl_sync(0xffffffffu, o, leader + t));
-        new_cost = __fadd_rn(new_cost, __shfl_sync(0xffffffffu, nw, leader + t));
-      }
-    } else {
-      const uint16_t gs1 = skip ? (uint16_t)0 : g1, gs2 = skip ? (uint16_t)0 : g2;
-      const float4 la1 = lab(gs1), la2 = lab(gs2);
-      // this lane's terms t = slot + kL * tt (0-3: neighbours of pos1 in up, down,
-      // left, right order; 4-7: those of pos2)
-      float o[kT], nw[kT], m[kT];
+      for (int h = 0; h < kWindow; h += 4) *reinterpret_cast<float4*>(d + h) = *reinterpret_cast<const float4*>(O.delta + h);
 #pragma unroll
-      for (int tt = 0; tt < kT; ++tt) {
-        const int t = slot + kL * tt;
-        const bool first = t < 4;
-        const int dir = t & 3;
-        const int bx = first ? x1 : x2, by = first ? y1 : y2;
-        const int nx = bx + (dir == 2 ? -1 : (dir == 3 ? 1 : 0)), ny = by + (dir == 0 ? -1 : (dir == 1 ? 1 : 0));
-        const bool inb = nx >= 0 && nx < gw && ny >= 0 && ny < gh;
-        const int nb = inb ? ny * gw + nx : p1;
-        const bool mutual = inb && nb == (first ? p2 : p1);
-        const uint16_t an = s_grid[nb];
-        const bool work = !skip && !same && inb;
-        const bool nbr = work && !mutual && an != kNone16;  // a placed neighbour
-        const uint16_t c_idx = mutual ? gs2 : (an != kNone16 ? an : gs1);
-        const float4 lc = lab(c_idx);
-        const float w1 = wgt(la1, lc), w2 = wgt(la2, lc);
-        o[tt] = nbr ? (first ? w1 : w2) : 0.0f;
-        nw[tt] = nbr ? (first ? w2 : w1) : 0.0f;
-        m[tt] = (work && mutual && first) ? w1 : 0.0f;
+      for (int h = 0; h < kWindow; ++h) {
+        current = __fadd_rn(current, d[h]);
+        d[h] = current;
       }
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        old_cost = __fadd_rn(old_cost, __shfl_sync(0xffffffffu, o[t / kL], leader + t % kL));
-        new_cost = __fadd_rn(new_cost, __shfl_sync(0xffffffffu, nw[t / kL], leader + t % kL));
+      for (int h = 0; h < kWindow; h += 4) *reinterpret_cast<float4*>(S.sums + h) = *reinterpret_cast<const float4*>(d + h);
+      __syncwarp();
+      float c[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t f = O.flags[32 * h + lane];
+        accepted += __popc(__ballot_sync(0xffffffffu, (f & 1u) != 0u));
+        cooled += __popc(__ballot_sync(0xffffffffu, (f & 2u) != 0u));
+        c[h] = S.sums[32 * h + lane];
       }
-      m0 = m[0];
-    }
-    const int dx = x2 - x1, dy = y2 - y1;
-    const bool adjacent = (dx == 0 && (dy == 1 || dy == -1)) || (dy == 0 && (dx == 1 || dx == -1));
-    const int dir12 = dy == -1 ? 0 : (dy == 1 ? 1 : (dx == -1 ? 2 : 3));
-    const float mm = __shfl_sync(0xffffffffu, m0, leader + dir12);  // term dir12 < 4 sits in lane dir12's first term
-    if (adjacent) {
-      old_cost = __fadd_rn(old_cost, mm);
-      new_cost = __fadd_rn(new_cost, mm);
-    }
-    const float delta = same ? 0.0f : __fsub_rn(new_cost, old_cost);
-    if (slot == 0) {
-      RoundSlot& r = s_round[q_mine];
-      r.delta = delta;
-      r.u = __int_as_float(e.z);
-      r.flags = skip ? 1u : 0u;
-      r.pos1 = (uint32_t)e.x;
-      r.pos2 = (uint32_t)e.y;
+      if (__any_sync(0xffffffffu, c[0] < best || c[1] < best)) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float least = c[h];  // of this lane's and the earlier ones
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_up_sync(0xffffffffu, least, o);
+            least = lane >= o ? fminf(least, v) : least;
+          }
+          float before = __shfl_up_sync(0xffffffffu, least, 1);
+          before = lane == 0 ? best : fminf(best, before);
+          improved += __popc(__ballot_sync(0xffffffffu, c[h] < before));
+          best = fminf(best, __shfl_sync(0xffffffffu, least, 31));
+        }
+      }
+      __syncwarp();
+    };
+    int slot = 0;
+    for (long long w = 0; w < windows; ++w) {
+      bar_sync(kBarFull + slot, kFullThreads);  // window w is prepared, the evaluators are in window w - 1
+      if (w > 1) book(S.out[(w - 2) % 3]);
+      slot = slot + 1 == kProducers ? 0 : slot + 1;
     }
     __syncthreads();
-
-    // ---- 2. the round's outcome, derived identically by every warp -------------------------
-    // lane q < kRound holds proposal q (lanes kRound.. duplicate lane q - kRound)
-    const int q = lane & (kRound - 1);
-    const RoundSlot rq = s_round[q];
-    const bool skip_q = rq.flags & 1u;
-    const unsigned live_mask = __ballot_sync(0xffffffffu, lane < kRound && !skip_q);  // bit q: not skipped
-    // The temperatures T_k (the chain's T after k more coolings, multiplied step
-    // by step); lane k keeps T_k.
-    // (T_kRound, wanted when every proposal of a 32-proposal round cools, is
-    // held by every lane as t_last: there is no lane 32)
-    float t_lane = temp, t_last = temp;
-    if (!greedy_only) {
-      float tk = temp;
-#pragma unroll
-      for (int kk = 1; kk <= kRound; ++kk) {
-        tk = __fmul_rn(tk, decay);
-        if (kk == lane) t_lane = tk;
-      }
-      t_last = tk;
+    if (windows > 1) book(S.out[(windows - 2) % 3]);
+    if (windows > 0) book(S.out[(windows - 1) % 3]);
+    if (lane == 0) {
+      ChainResult r;
+      r.initial_cost = initial;
+      r.final_cost = current;
+      r.best_cost = J.greedy_only ? current : best;
+      r.pad = 0.0f;
+      r.accepted = accepted;
+      r.improved = J.greedy_only ? accepted : improved;
+      r.cooled = cooled;
+      r.pad2 = 0;
+      J.results[chain] = r;
     }
-    bool acc_q = false;
-    {
-      const int before = __popc(live_mask & ((1u << q) - 1u));
-      const float t_q = __shfl_sync(0xffffffffu, t_lane, before);
-      if (!skip_q) {
-        if (greedy_only) acc_q = rq.delta < 0.0f;
-        else acc_q = rq.delta < 0.0f || rq.u < exp_spec(__fdiv_rn(-rq.delta, t_q));
-      }
-    }
-    const unsigned acc_mask = __ballot_sync(0xffffffffu, lane < kRound && acc_q);
-    // proposal q reads a cell within distance 1 of an earlier accepted swap?
-    // (branch-free: Manhattan distances of the four position pairs).  The
-    // earlier proposals h are split over the warps -- warp w tests
-    // h in [w * kConfPerWarp, (w + 1) * kConfPerWarp) for every q -- and the
-    // warps' conflict masks are ORed through shared memory.
-    const int qx1 = (int)(rq.pos1 & 0xFFFFu), qy1 = (int)(rq.pos1 >> 16);
-    const int qx2 = (int)(rq.pos2 & 0xFFFFu), qy2 = (int)(rq.pos2 >> 16);
-    unsigned conf_bits = 0u;
-#pragma unroll
-    for (int j = 0; j < kConfPerWarp; ++j) {
-      const int h = warp * kConfPerWarp + j;
-      const uint32_t hp1 = __shfl_sync(0xffffffffu, rq.pos1, h & 31), hp2 = __shfl_sync(0xffffffffu, rq.pos2, h & 31);
-      const int hx1 = (int)(hp1 & 0xFFFFu), hy1 = (int)(hp1 >> 16), hx2 = (int)(hp2 & 0xFFFFu), hy2 = (int)(hp2 >> 16);
-      const unsigned hit = (unsigned)(abs(hx1 - qx1) + abs(hy1 - qy1) <= 1) | (unsigned)(abs(hx1 - qx2) + abs(hy1 - qy2) <= 1) |
-                           (unsigned)(abs(hx2 - qx1) + abs(hy2 - qy1) <= 1) | (unsigned)(abs(hx2 - qx2) + abs(hy2 - qy2) <= 1);
-      conf_bits |= hit & (acc_mask >> (h & 31)) & (unsigned)(h < q);
-    }
-    const unsigned part = __ballot_sync(0xffffffffu, lane < kRound && (conf_bits & 1u) != 0u);
-    if (lane == 0) s_conf[warp] = part;
-    __syncthreads();
-    unsigned conf_mask = 0u;
-#pragma unroll
-    for (int w = 0; w < kChainWarps; ++w) conf_mask |= s_conf[w];
-    const unsigned cmask = conf_mask & live_mask;
-    const int gc = cmask ? __ffs(cmask) - 1 : kRound;  // >= 1: proposal 0 never conflicts
-    const int ncommit = (int)min((long long)gc, iters - it);
-    const unsigned commit = ncommit >= 32 ? 0xFFFFFFFFu : (1u << ncommit) - 1u;
-    // in-order bookkeeping (every thread, identical values)
-#pragma unroll
-    for (int h = 0; h < kRound; ++h) {
-      const float dh = __shfl_sync(0xffffffffu, rq.delta, h);
-      const bool a = ((acc_mask & commit) >> h) & 1u;
-      const float nc = __fadd_rn(current, dh);
-      current = a ? nc : current;
-      const bool imp = a && current < best;
-      best = imp ? current : best;
-      improved += imp ? 1 : 0;
-    }
-    accepted += __popc(acc_mask & commit);
-    const int ncool = __popc(live_mask & commit);  // skipped proposals do not cool
-    cooled += ncool;
-    if (!greedy_only) {
-      const float t_n = __shfl_sync(0xffffffffu, t_lane, ncool & 31);
-      temp = ncool == 32 ? t_last : t_n;
-    }
-    // ---- 3. committed accepted swaps -------------------------------------------------------
-    if (slot == 0 && q_mine < ncommit && ((acc_mask >> q_mine) & 1u)) {
-      s_grid[p1] = g2;
-      s_grid[p2] = g1;
-    }
-    it += ncommit;
-    __syncthreads();
   }
   int32_t* out = J.chain_grids + (size_t)chain * n;
   for (int i = tid; i < n; i += kThreads) {
     const uint16_t g = s_grid[i];
     out[i] = g == kNone16 ? -1 : (int32_t)g;
   }
-  if (tid == 0) {
-    ChainResult r;
-    r.initial_cost = initial;
-    r.final_cost = current;
-    r.best_cost = greedy_only ? current : best;
-    r.pad = 0.0f;
-    r.accepted = accepted;
-    r.improved = greedy_only ? accepted : improved;
-    r.cooled = cooled;
-    r.pad2 = 0;
-    J.results[chain] = r;
-  }
 }
 
-}  // namespace anneal_cta_detail
+}  // namespace anneal_detail
 }  // namespace mg

@@ -1,38 +1,21 @@
-// k_anneal.cu -- (e) the standalone annealing kernels (one CTA per chain,
-// anneal_cta.cuh; or one warp per chain, anneal_chain.cuh, for grids whose
-// state does not fit beside the CTA's round buffers) and the batched adjacency evaluators of the
-// C ABI (adjacency.rs:63-214), one thread per item, the reference's loops
-// verbatim.
+// k_anneal.cu -- (e) the annealing kernel (one CTA per chain, anneal_cta.cuh)
+// and the batched adjacency evaluators of the C ABI (adjacency.rs:63-214), one
+// thread per item, the reference's loops verbatim.
 #include "anneal_cta.cuh"
 
 namespace mg {
 namespace {
 using namespace anneal_detail;
 
-template <bool kLabSmem, int kRound>
-__global__ void __launch_bounds__(anneal_cta_detail::kThreads)
+template <bool kLabSmem, int kPerSm>
+__global__ void __launch_bounds__(kThreads, kPerSm)
     anneal_cta_kernel(const float4* __restrict__ pal, int p, const AnnealJob* __restrict__ jobs,
-                      const int* __restrict__ chain_job, const int* __restrict__ chain_id) {
+                      const int* __restrict__ chain_job, const int* __restrict__ chain_id, int writer_slots) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int jid = chain_job ? chain_job[blockIdx.x] : 0;
   const int chain = chain_id ? chain_id[blockIdx.x] : (int)blockIdx.x;
   const AnnealJob J = jobs[jid];
-  anneal_cta_detail::anneal_chain_cta<kLabSmem, kRound>(pal, p, J, chain, smem);
-}
-
-// Grids of at least this many cells take 32 proposals a round.
-constexpr int kWideRoundCells = 12000;
-
-template <bool kLabSmem>
-__global__ void __launch_bounds__(32) anneal_kernel(const float4* __restrict__ pal, int p,
-                                                    const AnnealJob* __restrict__ jobs,
-                                                    const int* __restrict__ chain_job,
-                                                    const int* __restrict__ chain_id) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  const int jid = chain_job ? chain_job[blockIdx.x] : 0;
-  const int chain = chain_id ? chain_id[blockIdx.x] : (int)blockIdx.x;
-  const AnnealJob J = jobs[jid];
-  anneal_chain<kLabSmem>(pal, p, J, chain, smem);
+  anneal_chain_cta<kLabSmem>(pal, p, J, chain, writer_slots, smem);
 }
 
 // Lowest final cost wins (ties: lowest chain); copy its grid.
@@ -146,52 +129,51 @@ __global__ void total_cost_kernel(const float4* __restrict__ pal, const int32_t*
 }  // namespace
 
 int launch_anneal(const float4* pal, int p, const AnnealJob* jobs_dev, const int* chain_job_dev,
-                  const int* chain_id_dev, int total_chains, int max_cells, cudaStream_t stream, int min_cells) {
+                  const int* chain_id_dev, int total_chains, int max_cells, cudaStream_t stream) {
   if (total_chains <= 0) return MG_OK;
   if (p >= 65535) return fail(MG_ERR_ARG, "annealing supports palettes below 65535 materials");
-  const size_t grid_bytes = kRing * sizeof(int4) + (((size_t)max_cells * 2 + 15) & ~(size_t)15);
-  const size_t lab_bytes = (size_t)p * sizeof(float4);
-  const size_t kMaxSmem = 200 * 1024;
-  if (grid_bytes > kMaxSmem) return fail(MG_ERR_ARG, "grid too large for the annealer (max 102400 cells)");
-  static int configured_device = -1;
+  // the grid alone may not pass 200 KB (the limit the calls document by their
+  // error); beside the chain's other state that always fits
+  constexpr size_t kMaxSmem = 226 * 1024;
+  if (max_cells > 101888) return fail(MG_ERR_ARG, "grid too large for the annealer (max 102400 cells)");
+  static int configured_device = -1, sms = 0;
   int dev = 0;
   MG_CUDA(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    MG_CUDA(cudaFuncSetAttribute(anneal_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    MG_CUDA(cudaFuncSetAttribute(anneal_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<true, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<false, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<true, 1>, a, (int)kMaxSmem));
+    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<false, 1>, a, (int)kMaxSmem));
+    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<true, 2>, a, (int)kMaxSmem));
+    MG_CUDA(cudaFuncSetAttribute(anneal_cta_kernel<false, 2>, a, (int)kMaxSmem));
+    MG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     configured_device = dev;
   }
-  // A CTA of several warps per chain (more proposals per round) when it fits.
-  {
-    using anneal_cta_detail::anneal_cta_smem_bytes;
-    const size_t with_lab = anneal_cta_smem_bytes(max_cells, p, true), no_lab = anneal_cta_smem_bytes(max_cells, p, false);
-    if (with_lab <= kMaxSmem || no_lab <= kMaxSmem) {
-      const bool wide = (min_cells < 0 ? max_cells : min_cells) >= kWideRoundCells;
-      const unsigned nt = anneal_cta_detail::kThreads;
-      if (with_lab <= kMaxSmem) {
-        if (wide)
-          anneal_cta_kernel<true, 32><<<total_chains, nt, with_lab, stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev);
-        else
-          anneal_cta_kernel<true, 16><<<total_chains, nt, with_lab, stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev);
-      } else {
-        if (wide)
-          anneal_cta_kernel<false, 32><<<total_chains, nt, no_lab, stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev);
-        else
-          anneal_cta_kernel<false, 16><<<total_chains, nt, no_lab, stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev);
-      }
-      g_launches += 1;
-      MG_CUDA(cudaGetLastError());
-      return MG_OK;
-    }
+  // One chain a multiprocessor (as many as there are, or fewer, chains): its
+  // latency counts, so all of shared memory goes to it -- the palette's Lab
+  // beside the grid, the rest to the writers table.  More chains than that
+  // (batches): two share a multiprocessor when they fit in half of it each,
+  // reading the Lab through L1 where it is too large for that.
+  constexpr size_t kHalfSmem = 113 * 1024;
+  const bool share = total_chains > sms && anneal_cta_smem_bytes(max_cells, p, false, kWriterSlotsShared) <= kHalfSmem;
+  const size_t room = share ? kHalfSmem : kMaxSmem;
+  int slots = share ? kWriterSlotsShared : kWriterSlots;
+  auto bytes = [&](bool lab) { return anneal_cta_smem_bytes(max_cells, p, lab, slots); };
+  auto shrink = [&](bool lab) {
+    while (slots > kWriterSlotsMin && bytes(lab) > room) slots >>= 1;
+    return bytes(lab) <= room;
+  };
+  const bool lab_smem = anneal_cta_smem_bytes(max_cells, p, true, kWriterSlotsShared) <= room;
+  if (!shrink(lab_smem)) return fail(MG_ERR_ARG, "grid too large for the annealer (max 102400 cells)");
+  auto go = [&](auto kernel) {
+    kernel<<<total_chains, kThreads, bytes(lab_smem), stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev, slots);
+  };
+  if (share) {
+    if (lab_smem) go(anneal_cta_kernel<true, 2>);
+    else go(anneal_cta_kernel<false, 2>);
+  } else {
+    if (lab_smem) go(anneal_cta_kernel<true, 1>);
+    else go(anneal_cta_kernel<false, 1>);
   }
-  if (grid_bytes + lab_bytes <= kMaxSmem)
-    anneal_kernel<true><<<total_chains, 32, grid_bytes + lab_bytes, stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev);
-  else
-    anneal_kernel<false><<<total_chains, 32, grid_bytes, stream>>>(pal, p, jobs_dev, chain_job_dev, chain_id_dev);
   g_launches += 1;
   MG_CUDA(cudaGetLastError());
   return MG_OK;
