@@ -392,7 +392,8 @@ __device__ __forceinline__ void evaluate_windows(const float4* __restrict__ pal,
 template <bool kLabSmem>
 __device__ __forceinline__ void anneal_chain_cta(const float4* __restrict__ pal, int p, const AnnealJob& J, int chain,
                                                  int writer_slots, uint8_t* smem) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the warp index through a shuffle: the compiler then knows each warp's path as converged
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int gw = J.gw, gh = J.gh, n = gw * gh;
   ChainShared& S = *reinterpret_cast<ChainShared*>(smem);
   uint32_t* writers = reinterpret_cast<uint32_t*>(smem + sizeof(ChainShared));

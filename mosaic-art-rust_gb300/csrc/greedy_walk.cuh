@@ -42,6 +42,7 @@
 #pragma once
 #include "mg_internal.h"
 #include "mg_ptx.cuh"
+#include "roots.cuh"
 
 namespace mg {
 namespace greedy_detail {
@@ -49,10 +50,6 @@ namespace greedy_detail {
 constexpr int kStageCells = 16;  // cells per TMA stage (candidate rows are k entries each)
 constexpr int kStageBufs = 4;    // stages in flight
 constexpr uint32_t kNoCand = 0xFFFFFFFFu;
-
-__device__ __forceinline__ float wgt(const float4& a, const float4& b) {
-  return __frcp_rn(__fadd_rn(lab_distance(a.x, a.y, a.z, b.x, b.y, b.z), 1.0f));
-}
 
 // Sequential calculate_total_cost of a complete grid by one warp: lanes compute
 // the right and down terms of 32 cells, lane order then feeds one FP32

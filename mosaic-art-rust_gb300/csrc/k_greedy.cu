@@ -12,33 +12,45 @@
 //    whose three-CTA form does not fit in shared memory.
 //  - greedy_pair_kernel: a cluster of three CTAs per mosaic.  The walk is a
 //    chain of dependent decisions, so its speed is the latency of one decision.
-//    One warp of CTA 0 (the walker) makes the decisions; 64 scout warps in
-//    CTAs 1 and 2, on other SMs, prepare each cell's decision ahead of the walker
-//    from a snapshot of the usage counters, reading the walk's state and
-//    writing their records through distributed shared memory:
-//      the first 32 candidates (list order) that differ from the cell above
-//      and were under the usage cap in the snapshot, and for each whether the
-//      next such candidate lies outside its 2*weight window (`clear`: then the
-//      penalty cannot change the decision if that candidate is the first
-//      eligible one); also the first 32 candidates regardless of the counters,
-//      for use after a reset.
-//    Counters only grow between resets, so a candidate that failed the cap in
-//    the snapshot still fails it when the walker arrives: the walker's first
-//    eligible candidate is the first record entry that passes the fresh
-//    counter and differs from the left neighbour -- one warp minimum -- and
-//    with its `clear` bit set it is the reference's choice, bit for bit.  In
-//    every other case (window not clear, no entry passes, a reset since the
-//    snapshot for the filtered list) the walker evaluates the cell in full,
-//    exactly as greedy_walk does -- except that with the palette Lab in global
-//    memory a window that closes inside the filtered list is settled from the
-//    record (window_cell).  A scout builds a record once the walker has placed
-//    the cell kLead cells (or a row) back, polling the walker's ring of
-//    placed cells, and a reset bumps an epoch that invalidates older snapshots.
-//    The walker's shared memory holds rings (records, placed cells), not the
-//    grid, so a mosaic of any cell count walks in this form.  After the walk
-//    the scout CTA computes calculate_total_cost: terms in parallel, one
-//    sequential FP32 sum in the reference's order.
+//    One warp of CTA 0 (the walker) makes them; everything that does not depend
+//    on the last few is prepared ahead of it, in two steps:
+//    * 62 scout warps in CTAs 1 and 2, on other SMs, turn each cell's candidate
+//      row into a record, kScoutLead cells ahead: the first 32 candidates (list
+//      order) that differ from the cell above and were under the usage cap in a
+//      snapshot of the counters (a copy that a follower warp keeps in each of
+//      those CTAs), with distance, Lab and weight against the cell above; also
+//      the first 32 candidates regardless of the counters, for use after a reset;
+//    * kRefiners warps of CTA 0 turn each record into a list of eight entries,
+//      kRefineLag cells ahead, from the counters themselves (see ListShared).
+//    Counters only grow between resets, so a candidate that failed the cap in a
+//    snapshot still fails it when the walker arrives: the walker's choice is the
+//    list entry of lowest rank that passes the fresh counter and is not the left
+//    neighbour's material -- one warp minimum -- whenever the list settles it,
+//    bit for bit the reference's.  In every other case (nothing of the list
+//    passes, something beyond it might win, a reset since the snapshot) the
+//    walker decides from the record (window_cell) or evaluates the cell in full,
+//    exactly as greedy_walk does.  A reset bumps an epoch that invalidates older
+//    records and lists.  Where the 16-bit grid does not fit, the walker's shared
+//    memory holds a ring of the last placed cells instead, so a mosaic of any
+//    cell count walks in this form.  calculate_total_cost: by a warp of CTA 0
+//    that follows the walk (with the ring: by CTA 1 after it), one sequential
+//    FP32 sum in the reference's order.
+//
+//    What bounds it: the walker's loop, ~100 cycles a cell (the minimum 22, the
+//    rotation, test and exclusion before it ~20, two branches ~40), and lists
+//    that are not there in time: ~500 cycles from trigger to list, ~1 000 when
+//    penalties decide.  Measured, GB300, before (records alone, no lists; 64
+//    scouts that read the counters through distributed shared memory) -> now:
+//    80 x 60 cells, 506 materials 0.551 -> 0.348 ms; 179 x 134, 5000 materials
+//    3.49 -> 1.78; 61 x 43, 112 materials, cap 2 0.518 -> 0.274; 64 mosaics of
+//    300 to 17 900 cells, 10 000 materials 4.6 -> 1.68.  Measured and not kept:
+//    blocks of 2 or 4 cells without branches (80 cycles a cell alone, but a list
+//    that is late costs a whole block), lists made 10, 14 or 20 cells ahead (late;
+//    or, with caps of 2, filled before they are used), 11 or 20 refiners (too
+//    few; or in each other's way), refiners on the walker's scheduler, 124
+//    scouts, counters gathered two rounds at once.
 #include <cstddef>
+#include <type_traits>
 
 #include "greedy_walk.cuh"
 
@@ -58,26 +70,23 @@ __global__ void __launch_bounds__(32) greedy_kernel(const float4* __restrict__ p
 
 // ---- the scouted walk -------------------------------------------------------------------
 // A cluster of 1 + kScoutCtas CTAs per mosaic.  CTA 0 walks (warp 0; the
-// state of the walk lives in its shared memory); the other CTAs, on other
-// SMs, hold the scouts, which read the walk's state and write their records
-// through distributed shared memory, so the walker's SM runs nothing but the
-// walk.  Two cluster shapes hold the same 64 scouts: four scout CTAs of 16
-// warps (128 registers a thread, which the walker's loop uses: a launch of a
-// few mosaics), or two of 32 warps (64 registers; a batch, whose clusters
-// then take three SMs each instead of five).
-constexpr int kScouts = 64;                 // every warp of the scout CTAs
-constexpr int kScoutWarpsMax = 32;          // per CTA, the larger shape
+// state of the walk lives in its shared memory) with the refiners on its other
+// schedulers; the other CTAs, on other SMs, hold the scouts and a follower each
+// that copies the walk for them, so the walker's SM is read by one warp of each
+// and written the records, through distributed shared memory.  (Four scout CTAs
+// gained nothing over two.)
+constexpr int kScoutCtas = 2;
+constexpr int kThreads = 1024;      // per CTA
+constexpr int kScoutWarpsMax = 32;  // warps of a scout CTA
 constexpr uint32_t kInvalidEpoch = 0xFFFFFFFFu;
 constexpr uint32_t kWalkPolls = 1u << 24;      // the walker's bounded wait for a record
 constexpr uint32_t kInjectedWalkPolls = 1u << 12;  // ... when a timeout is injected (well under a millisecond)
-constexpr uint32_t kScoutPolls = 1u << 22;  // polls of about 1 us each
-// Records are built at most kLead cells ahead of the walker: 124 in the
-// five-CTA shape (a ring of 128 holds them; fewer late records), 80 in the
-// three-CTA shape of batches (fresher snapshots: fewer cells whose whole list
-// was capped since, which matters with their dense palettes).  The rings are
-// sized for the larger.
-constexpr int kScoutLead = 124;
-constexpr int kScoutLeadBatch = 80;
+constexpr uint32_t kScoutPolls = 1u << 24;  // polls of about 0.3 us each
+// Records are built at most kScoutLead cells ahead of the walker: far enough
+// that they are there in time, and no further, as every placement made since a
+// snapshot may have filled one of its entries.
+constexpr int kScoutLead = 80;
+constexpr uint32_t kRefinePolls = 1u << 26;  // the refiners' bounded waits (seconds)
 constexpr int kCostChunk = 2048;  // cells per pass of the final cost sum
 constexpr uint32_t kFollowPolls = 1u << 26;  // the cost warp's bounded wait for a placement (seconds)
 enum Ctrl { kProgress = 0, kEpoch = 1, kAbort = 2 };
@@ -145,26 +154,97 @@ __host__ __device__ inline int cell_ring_size(int gw) {
 }
 __device__ __forceinline__ uint32_t cell_word(int c, int t) { return ((uint32_t)c << 16) | ((uint32_t)t & 0xFFFFu); }
 
-// Shared memory of the walker CTA: control words, record ring, sequence
-// words, the placed cells (grid or ring), usage counters, optionally the
-// palette Lab.
+// The prepared lists.  Beside the walker (warp 0), refiner warps of its CTA --
+// none on the walker's scheduler -- turn each cell's record into what the
+// decision needs last, kRefineLag cells ahead of the walker: the first kList
+// entries under the usage cap *now* (a record's snapshot is up to kLead
+// placements old).  A list is written in list (= distance) order first, each
+// entry with whether the next one lies outside its 2*weight window: then, if it
+// is the first that may be taken, the penalty cannot change the decision.  When
+// every entry is clear like that, the list is done.  Else a second form follows,
+// ~500 cycles later: each entry's rank by score (then position), given each
+// entry of the previous cell's list as the left neighbour -- the one part of a
+// score not known before.  (When one of the first kEarly entries is not clear,
+// the second form is the only one.)
+// An entry of a list is one 64-bit word:
+//   low:  eight 4-bit ranks, rotated so that a left rotation by 4 j + 2 brings
+//         the one for previous entry j to the top (first form: the position):
+//         15 when the entry is absent, 14 when its score exceeds the distance
+//         of the first entry after the list (something beyond it might win);
+//   high: epoch (its low bits, list_tag) << 28 | position << 25 | clear << 24 | parity of the
+//         cell's turn of the ring << 23 | 1 << 16 | material (p when absent).
+// With j known from the previous decision the walker's choice is one warp
+// minimum over (rank, position, counter, material) of the entries still under
+// the cap and not the left neighbour's material: entries after a list have
+// distances, and so scores, of at least the first one's distance, so an entry
+// of score up to that is the reference's choice (ties go to the lower position).
+constexpr int kList = 8;
+constexpr int kRefiners = 17;   // warps 2, 3, 5, 6, 7, 9, ... of the walker's CTA
+constexpr int kRefineLag = 12;
+constexpr int kEarly = 3;       // entries that must be clear for the first form (2 to 8 differ by 3%)
+constexpr int kLists = 16;      // ring of lists (more than kRefineLag + 3)
+constexpr uint32_t kRankOpen = 14, kClear = 1u << 24;
+constexpr uint32_t kNotThere = 0xFFFFu;  // the packed word of an entry whose list is not there
+constexpr int kResetLog = 256;  // more resets than cells between the walker and its followers
+// The tag bits of a list: a slot holds cell c's list or still the one a turn of
+// the ring before; between a list's making and its use lie fewer than 32 cells,
+// so fewer than 32 resets.
+constexpr uint32_t kTagMask = 0xF0820000u, kTagCell = 0x00800000u;
+__device__ __forceinline__ uint32_t list_tag(int c, uint32_t epoch) {
+  return (epoch << 28) | ((epoch & 16u) << 13) | (((uint32_t)c & kLists) ? kTagCell : 0u);
+}
+static_assert((kLists & (kLists - 1)) == 0 && kLists <= 32 && kRefineLag + 4 <= kLists, "the list ring");
+struct __align__(16) ListShared {
+  unsigned long long ent[kLists][kList];  // first form
+  unsigned long long fin[kLists][kList];  // second form
+  unsigned long long spare[2];      // written where an entry has no place
+  uint32_t done[kLists];         // cell + 1 once all of its lists are written
+  float4 sel[kLists][kList + 1];    // Lab, material bits (the last one: what the list does not take)
+  uint32_t seq[kLists];             // cell + 1 once sel is complete
+  float2 dw[kRefiners][kList + 1];  // distance, weight against the cell above
+  uint32_t reset_at[kResetLog];     // the cell that began epoch e, at e % kResetLog
+};
+static_assert(sizeof(ListShared) % 16 == 0, "16-byte aligned parts");
+
+// Shared memory of the walker CTA: control words, lists, record ring, sequence
+// words, the placed cells (grid or ring), usage counters (and one more, full, for
+// absent entries), optionally the palette Lab.
 __host__ __device__ inline size_t cells_bytes(int gw, int n, bool ring) {
   return ring ? (size_t)cell_ring_size(gw) * 4 : align16((size_t)n * 2);
 }
 __host__ __device__ inline size_t walker_smem_bytes(int gw, int n, int p, bool lab_smem, bool ring) {
   const int R = ring_size(gw);
-  size_t b = 16 + (size_t)R * sizeof(CellRecord) + (size_t)R * 4;
+  size_t b = 16 + sizeof(ListShared) + (size_t)R * sizeof(CellRecord) + (size_t)R * 4;
   b += cells_bytes(gw, n, ring);
-  b += align16((size_t)p * 4);
+  b += align16(((size_t)p + 1) * 4);
   if (lab_smem) b += (size_t)p * 16;
   return b;
 }
-// Shared memory of the scout CTA: staging per warp, then the cost terms.
-__host__ __device__ inline size_t scout_cta_smem_bytes() {
-  return (size_t)kScoutWarpsMax * sizeof(ScoutStage) + (size_t)kCostChunk * 8;
+// Shared memory of a scout CTA: staging per warp, the cost terms, and its copy
+// of the walk (follow_walk): control words, counters, the last placed cells.
+struct ScoutLayout {
+  ScoutStage* stage;
+  float* terms;
+  uint32_t* ctl;  // Follow
+  uint32_t* usage;
+  uint16_t* cells;  // ring of cell_ring_size(gw)
+};
+enum Follow { kFollowed = 0, kFollowEpoch = 1, kFollowAbort = 2 };
+__device__ inline ScoutLayout scout_layout(uint8_t* smem, int p) {
+  ScoutLayout S;
+  S.stage = reinterpret_cast<ScoutStage*>(smem);
+  S.terms = reinterpret_cast<float*>(S.stage + kScoutWarpsMax);
+  S.ctl = reinterpret_cast<uint32_t*>(S.terms + 2 * kCostChunk);
+  S.usage = S.ctl + 4;
+  S.cells = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(S.usage) + align16((size_t)p * 4));
+  return S;
+}
+__host__ __device__ inline size_t scout_cta_smem_bytes(int gw, int p) {
+  return (size_t)kScoutWarpsMax * sizeof(ScoutStage) + (size_t)kCostChunk * 8 + 16 + align16((size_t)p * 4) +
+         (size_t)cell_ring_size(gw) * 2;
 }
 __host__ __device__ inline size_t pair_smem_bytes(int gw, int n, int p, bool lab_smem, bool ring) {
-  const size_t a = walker_smem_bytes(gw, n, p, lab_smem, ring), b = scout_cta_smem_bytes();
+  const size_t a = walker_smem_bytes(gw, n, p, lab_smem, ring), b = scout_cta_smem_bytes(gw, p);
   return a > b ? a : b;
 }
 
@@ -174,7 +254,7 @@ __host__ __device__ inline size_t pair_smem_bytes(int gw, int n, int p, bool lab
 template <class LabFn>
 __device__ int full_cell(LabFn lab, const uint32_t* __restrict__ ci, const float* __restrict__ cd, int k, int p, int up,
                          int left, uint32_t* usage, uint32_t max_usage, float weight, uint32_t* ctrl,
-                         uint32_t& epoch, int& resets, int lane) {
+                         uint32_t& epoch, int& resets, int lane, uint32_t* reset_at, int c) {
   const bool use_pen = weight > 0.0f;
   const float two_w = __fmul_rn(2.0f, weight);
   auto okf = [&](uint32_t t, int j) {
@@ -256,6 +336,7 @@ __device__ int full_cell(LabFn lab, const uint32_t* __restrict__ ci, const float
     ++epoch;
     if (lane == 0) {
       usage[t] = 1u;
+      reset_at[epoch % kResetLog] = (uint32_t)c;
       st_release_cluster(smem_u32(&ctrl[kEpoch]), epoch);
     }
   }
@@ -270,7 +351,7 @@ __device__ int full_cell(LabFn lab, const uint32_t* __restrict__ ci, const float
 template <class LabFn>
 __device__ int full_cell_rows(LabFn lab, const uint32_t* __restrict__ ci, const float* __restrict__ cd, int k, int p,
                               int up, int left, uint32_t* usage, uint32_t max_usage, float weight, uint32_t* ctrl,
-                              uint32_t& epoch, int& resets, int lane) {
+                              uint32_t& epoch, int& resets, int lane, uint32_t* reset_at, int c) {
   constexpr int kRounds = 4;  // ceil(100 / 32)
   const bool use_pen = weight > 0.0f;
   const float two_w = __fmul_rn(2.0f, weight);
@@ -364,6 +445,7 @@ __device__ int full_cell_rows(LabFn lab, const uint32_t* __restrict__ ci, const 
     ++epoch;
     if (lane == 0) {
       usage[t] = 1u;
+      reset_at[epoch % kResetLog] = (uint32_t)c;
       st_release_cluster(smem_u32(&ctrl[kEpoch]), epoch);
     }
   }
@@ -374,6 +456,7 @@ __device__ int full_cell_rows(LabFn lab, const uint32_t* __restrict__ ci, const 
 // it into the walker CTA's window).
 struct WalkerLayout {
   uint32_t* ctrl;
+  ListShared* lists;
   CellRecord* rec;
   uint32_t* seq;
   uint32_t* ring;    // the placed cells as a ring (kRing) ...
@@ -384,13 +467,86 @@ struct WalkerLayout {
 __device__ inline WalkerLayout walker_layout(uint8_t* smem, int gw, int n, int p, int R, bool ring) {
   WalkerLayout L;
   L.ctrl = reinterpret_cast<uint32_t*>(smem);
-  L.rec = reinterpret_cast<CellRecord*>(smem + 16);
+  L.lists = reinterpret_cast<ListShared*>(smem + 16);
+  L.rec = reinterpret_cast<CellRecord*>(L.lists + 1);
   L.seq = reinterpret_cast<uint32_t*>(L.rec + R);
   L.ring = L.seq + R;
   L.grid16 = reinterpret_cast<uint16_t*>(L.ring);
   L.usage = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(L.ring) + cells_bytes(gw, n, ring));
-  L.lab = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(L.usage) + align16((size_t)p * 4));
+  L.lab = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(L.usage) + align16(((size_t)p + 1) * 4));
   return L;
+}
+
+// The follower warp of a scout CTA keeps a copy of the walk in that CTA's shared
+// memory: the cells placed so far, the counters, the epoch.  The scouts then
+// read nothing from the walker's SM -- gathering up to a hundred counters there
+// for every cell kept its shared memory busier than the walk did, and a scout
+// 5 us a cell (64 scouts: 175 cycles a cell).  The copy lags; counters that lag
+// only list entries that are full by now, and an epoch that lags only makes the
+// record one of the earlier epoch.
+template <bool kRing>
+__device__ void follow_walk(const GreedyJob& J, int p, uint8_t* smem, int R, uint32_t* err) {
+  const int lane = threadIdx.x & 31;
+  const int gw = J.gw, n = gw * J.gh;
+  const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
+  const ScoutLayout S = scout_layout(smem, p);
+  const uint32_t r_epoch = cluster_map(&L.ctrl[kEpoch], 0), r_abort = cluster_map(&L.ctrl[kAbort], 0);
+  const uint32_t r_cells = cluster_map(L.ring, 0), r_log = cluster_map(L.lists->reset_at, 0);
+  const int cmask = cell_ring_size(gw) - 1;
+  uint32_t mine = 0, polls = 0;
+  for (int pos = 0; pos < n;) {
+    const int cc = pos + lane;
+    uint32_t v = 0;
+    bool placed = false;
+    if (cc < n) {
+      v = kRing ? ld_cluster_u32(r_cells + 4u * (uint32_t)(cc & cmask)) : ld_cluster_u16(r_cells + 2u * (uint32_t)cc);
+      placed = kRing ? (v >> 16) == ((uint32_t)cc & 0xFFFFu) : v != kUnplaced;
+      v &= 0xFFFFu;
+    }
+    const unsigned missing = __ballot_sync(0xffffffffu, !placed);
+    const int run = missing ? __ffs(missing) - 1 : 32;
+    if (run == 0) {
+      const bool out = ++polls > kScoutPolls;
+      if (__any_sync(0xffffffffu, out || ld_cluster_u32(r_abort) != 0u)) {
+        if (lane == 0) {
+          if (out) {
+            atomicOr(err, kErrTimeout);
+            st_cluster_u32(r_abort, 1u);
+          }
+          *reinterpret_cast<volatile uint32_t*>(&S.ctl[kFollowAbort]) = 1u;
+        }
+        return;
+      }
+      __nanosleep(100);
+      continue;
+    }
+    polls = 0;
+    const uint32_t epoch = __shfl_sync(0xffffffffu, ld_acquire_cluster(r_epoch), 0);
+    int from = 0;  // the run's cells before it are counted
+    while (mine != epoch) {
+      const int at = (int)__shfl_sync(0xffffffffu, ld_cluster_u32(r_log + 4u * ((mine + 1u) % kResetLog)), 0);
+      if (at >= pos + run) break;  // not there yet
+      if (lane == 0) st_release_cta(&S.ctl[kFollowEpoch], kInvalidEpoch);
+      __threadfence_block();
+      __syncwarp();
+      for (int i = lane; i < p; i += 32) S.usage[i] = 0;
+      __syncwarp();
+      // (a reset seen late: the cells counted since it)
+      for (int i = at + lane; i < pos; i += 32) atomicAdd(&S.usage[S.cells[i & cmask]], 1u);
+      from = max(from, at - pos);
+      __threadfence_block();
+      __syncwarp();
+      ++mine;
+      if (lane == 0) st_release_cta(&S.ctl[kFollowEpoch], mine);
+      __syncwarp();
+    }
+    if (lane >= from && lane < run) atomicAdd(&S.usage[v], 1u);
+    if (lane < run) S.cells[cc & cmask] = (uint16_t)v;
+    __syncwarp();
+    pos += run;
+    if (lane == 0) st_release_cta(&S.ctl[kFollowed], (uint32_t)pos);
+    __syncwarp();
+  }
 }
 
 // A scout warp: prepares the records of cells s, s + kScouts, s + 2 kScouts, ...
@@ -400,22 +556,21 @@ __device__ inline WalkerLayout walker_layout(uint8_t* smem, int gw, int n, int p
 // generic ones.)
 // withhold: build the records but never publish them (an injected fault: the
 // walker's wait for the first record then runs out).
-template <bool kRing, int kLead>
+template <bool kRing, int kLead, int kScouts>
 __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict__ pal, int p, uint8_t* smem,
                             ScoutStage& S, int R, uint32_t* err, bool withhold) {
   const int lane = threadIdx.x & 31;
   const int gw = J.gw, k = J.k, n = gw * J.gh;
   const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
+  const ScoutLayout F = scout_layout(smem, p);
   const uint32_t max_usage = J.max_usage;
   const bool use_pen = J.weight > 0.0f;
   const float two_w = __fmul_rn(2.0f, J.weight);
   const int nr = (k + 31) >> 5;
   const float inf = __int_as_float(0x7f800000);
   const unsigned lt = (1u << lane) - 1u;
-  // the walker CTA's words, in the cluster window
-  const uint32_t r_epoch = cluster_map(&L.ctrl[kEpoch], 0), r_abort = cluster_map(&L.ctrl[kAbort], 0);
-  const uint32_t r_usage = cluster_map(L.usage, 0), r_cells = cluster_map(L.ring, 0);
   const int cmask = cell_ring_size(gw) - 1;
+  // the walker CTA's records, in the cluster window
   const uint32_t r_rec = cluster_map(L.rec, 0), r_seq = cluster_map(L.seq, 0);
   for (int c = s; c < n; c += kScouts) {
     const int y = c / gw;
@@ -433,54 +588,35 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
         d[r] = __ldg(cd + j);
       }
     }
-    // Wait until the walker has placed cell c - min(gw, kLead): the
-    // cell above is then placed, and the counters this record is filtered by
-    // are at most kLead placements old (in a region of one colour a
-    // row's placements cap dozens of the nearest materials; a record built a
-    // whole row ahead would list none left).  Each cell is written once, by a
-    // single 16-bit store, so a scout that sees a value sees the final one; and
-    // the walker read that cell's record before placing it (the placement
-    // depends on it), so the walker is done with the ring slot this record
-    // reuses (the ring holds more than gw records).
+    // Wait until the follower has cell c - min(gw, kLead): the cell above is
+    // then known, and the counters this record is filtered by are at most kLead
+    // placements (and the follower's lag) old (in a region of one colour a row's
+    // placements cap dozens of the nearest materials; a record built a whole
+    // row ahead would list none left).  The walker read that cell's record
+    // before placing it (the placement depends on it), so the walker is done
+    // with the ring slot this record reuses (the ring holds more than gw records).
     const int lead = c - min(gw, kLead);
-    uint32_t v_lead = kNoCell;  // the lead cell's material in the low 16 bits
-    if (lead >= 0) {
-      const uint32_t a_lead = kRing ? r_cells + 4u * (uint32_t)(lead & cmask) : r_cells + 2u * (uint32_t)lead;
-      const uint32_t tag = (uint32_t)lead & 0xFFFFu;
-      uint32_t polls = 0;
-      auto placed = [&]() {
-        if (kRing) {
-          v_lead = ld_cluster_u32(a_lead);
-          return (v_lead >> 16) == tag;
+    for (uint32_t polls = 0;
+         lead >= 0 && !__all_sync(0xffffffffu, (int)ld_acquire_cta(&F.ctl[kFollowed]) > lead);) {
+      const bool out = ++polls > kScoutPolls;
+      if (__any_sync(0xffffffffu, out || ld_volatile_u32(&F.ctl[kFollowAbort]) != 0u)) {
+        if (out && lane == 0) {
+          atomicOr(err, kErrTimeout);
+          st_cluster_u32(cluster_map(&L.ctrl[kAbort], 0), 1u);
         }
-        v_lead = ld_cluster_u16(a_lead);
-        return v_lead != kUnplaced;
-      };
-      while (!placed()) {
-        if (ld_cluster_u32(r_abort)) return false;
-        if (++polls > kScoutPolls) {
-          if (lane == 0) {
-            atomicOr(err, kErrTimeout);
-            st_cluster_u32(r_abort, 1u);
-          }
-          return false;
-        }
-        __nanosleep(1000);  // the scouts run far ahead: poll the walker's SM rarely
+        return false;
       }
+      __nanosleep(100);
     }
-    const int up = y == 0           ? -1
-                   : lead == c - gw ? (int)(v_lead & 0xFFFFu)
-                   : kRing          ? (int)(ld_cluster_u32(r_cells + 4u * (uint32_t)((c - gw) & cmask)) & 0xFFFFu)
-                                    : (int)ld_cluster_u16(r_cells + 2u * (uint32_t)(c - gw));
-    const uint32_t ep0 = ld_acquire_cluster(r_epoch);
+    const int up = y == 0 ? -1 : (int)*reinterpret_cast<const volatile uint16_t*>(&F.cells[(c - gw) & cmask]);
+    const uint32_t ep0 = ld_acquire_cta(&F.ctl[kFollowEpoch]);
     int bf = 0, br = 0;
     float af = inf, ar = inf;  // distance of the 33rd entry
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (r < nr && (bf <= 32 || br <= 32)) {
         const bool in = t[r] < (uint32_t)p && (int)t[r] != up;
-        // counters are read on demand: each one is a load from the walker's SM
-        const bool okf = in && ld_cluster_u32(r_usage + 4u * t[r]) < max_usage;
+        const bool okf = in && ld_volatile_u32(&F.usage[t[r]]) < max_usage;
         const unsigned mf = __ballot_sync(0xffffffffu, okf), mr = __ballot_sync(0xffffffffu, in);
         const int pf = bf + __popc(mf & lt), pr = br + __popc(mr & lt);
         if (okf && pf < 32) {
@@ -499,8 +635,8 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
         br += __popc(mr);
       }
     }
-    fence_cluster();
-    const uint32_t ep1 = ld_acquire_cluster(r_epoch);
+    __threadfence_block();
+    const uint32_t ep1 = ld_acquire_cta(&F.ctl[kFollowEpoch]);
     __syncwarp();
     const int cf = min(bf, 32), cr = min(br, 32);
     // static window test of entry `lane` against the next entry of its list
@@ -547,22 +683,224 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
   return true;
 }
 
-template <bool kLabSmem, bool kRing, int kScoutCtas, int kWarps>
-__global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWarps * 32))
+// Refiner r: prepares the lists of cells r, r + kRefiners, ...  Every wait is
+// bounded; one that runs out aborts the walk.
+template <bool kLabSmem, bool kRing>
+__device__ void refine_cells(int r, const GreedyJob& J, const float4* __restrict__ pal, int p, uint8_t* smem, int R,
+                             uint32_t* err) {
+  const int lane = threadIdx.x & 31;
+  const int gw = J.gw, k = J.k, n = gw * J.gh;
+  const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
+  ListShared& Q = *L.lists;
+  const float4* s_lab = L.lab;
+  auto lab = [&](int i) -> float4 { return kLabSmem ? s_lab[i] : __ldg(pal + i); };
+  const int cmask = cell_ring_size(gw) - 1;
+  const uint32_t max_usage = J.max_usage;
+  const float weight = J.weight, two_w = __fmul_rn(2.0f, weight), inf = __int_as_float(0x7f800000);
+  const bool use_pen = weight > 0.0f;
+  const unsigned lt = (1u << lane) - 1u;
+  const int i = lane & 7, j0 = lane >> 3;
+  // polls until ok() in every lane; false (in every lane): aborted
+  auto wait = [&](auto ok) -> bool {
+    for (uint32_t polls = 0; !__all_sync(0xffffffffu, ok());) {
+      if ((++polls & 15u) == 0u) {
+        const bool out = polls > kRefinePolls;
+        if (__any_sync(0xffffffffu, out || ld_volatile_u32(&L.ctrl[kAbort]) != 0u)) {
+          if (out && lane == 0) {
+            atomicOr(err, kErrTimeout);
+            *reinterpret_cast<volatile uint32_t*>(&L.ctrl[kAbort]) = 1u;
+          }
+          return false;
+        }
+      }
+    }
+    return true;
+  };
+  auto at = [&](int c) -> uint32_t {  // a placed cell's material
+    return kRing ? ld_volatile_u32(&L.ring[c & cmask]) & 0xFFFFu
+                 : (uint32_t)*reinterpret_cast<const volatile uint16_t*>(&L.grid16[c]);
+  };
+  const uint32_t usage0 = smem_u32(L.usage);
+  // Whether the record of cell c (this warp's) is published; a probe looks at
+  // the warp's next 8 (lane l at cell c + l * kRefiners).
+  int ready_until = 0;
+  auto published = [&](int c) -> bool {
+    if (c < ready_until) return true;
+    const int cc = c + (lane & 7) * kRefiners;
+    const bool mine = cc >= n || ld_acquire_cluster(smem_u32(&L.seq[cc & (R - 1)])) == (uint32_t)(cc + 1);
+    const unsigned no = __ballot_sync(0xffffffffu, !mine) & 0xFFu;
+    ready_until = c + (no ? __ffs(no) - 1 : 8) * kRefiners;
+    return c < ready_until;
+  };
+  // A cell's candidates, one a lane: the record's list, or, when it is of an
+  // earlier epoch, the first 32 candidates of the row.  m = p: none.
+  uint32_t m = (uint32_t)p, rec_epoch = 0;
+  float d = inf, after = inf, wu = 0.0f;
+  float4 la = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto load_row = [&](int c) {
+    const uint32_t* ci = J.cand_idx + (size_t)c * k;
+    const float* cd = J.cand_dist + (size_t)c * k;
+    m = lane < k ? __ldg(ci + lane) : kNoCand;
+    d = lane < k ? __ldg(cd + lane) : inf;
+    after = k > 32 ? __ldg(cd + 32) : inf;
+    const int up = c >= gw ? (int)at(c - gw) : -1;
+    if ((int)m == up || m >= (uint32_t)p) m = (uint32_t)p;
+    wu = 0.0f;
+    la = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (m < (uint32_t)p) {
+      la = lab((int)m);
+      if (use_pen && up >= 0) wu = wgt(la, lab(up));
+    }
+  };
+  bool use_f = false;
+  auto load_record = [&](int c) {
+    const CellRecord& Rc = L.rec[c & (R - 1)];
+    rec_epoch = Rc.epoch;
+    const uint32_t key = Rc.kf[lane];
+    m = key == 0xFFFFFFFFu ? (uint32_t)p : key & 0xFFFFu;
+    d = Rc.wd[lane];
+    wu = Rc.wu[lane];
+    la = Rc.wl[lane];
+    after = Rc.f_next;
+  };
+  int x = r % gw;
+  bool have = false;  // the cell's record is read
+  for (int c = r; c < n; c += kRefiners) {
+    const int slot = c & (kLists - 1);
+    if (!have) {
+      if (!wait([&] { return published(c); })) return;
+      load_record(c);
+    }
+    // the slot is free: its last cell's lists are done, and the next cell's,
+    // which reads this one's (the walker may have passed both on first forms)
+    const int past = c - kLists;
+    if (past >= 0 && !wait([&] {
+          return (int)ld_acquire_cta(&Q.done[slot]) > past &&
+                 (int)ld_acquire_cta(&Q.done[(past + 1) & (kLists - 1)]) > past + 1;
+        }))
+      return;
+    use_f = __all_sync(0xffffffffu, rec_epoch == ld_volatile_u32(&L.ctrl[kEpoch]));
+    if (!use_f) load_row(c);
+    const int lead = c - kRefineLag;
+    if (lead >= 0 && !wait([&] {
+          return kRing ? (ld_volatile_u32(&L.ring[lead & cmask]) >> 16) == ((uint32_t)lead & 0xFFFFu)
+                       : at(lead) != kUnplaced;
+        }))
+      return;
+    // the epoch, then the counters: they only grow within an epoch, so an entry
+    // at the cap now stays there
+    const uint32_t epoch = ld_acquire_cta(&L.ctrl[kEpoch]);
+    auto counter = [&] {
+      uint32_t u;
+      asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(u) : "r"(usage0 + 4u * m) : "memory");
+      return u;
+    };
+    uint32_t used = counter();
+    if (use_f && __any_sync(0xffffffffu, rec_epoch != epoch)) {  // a reset while it waited
+      load_row(c);
+      used = counter();
+    }
+    const bool under = used < max_usage;
+    const unsigned um = __ballot_sync(0xffffffffu, under);
+    const int cnt = __popc(um), rk = __popc(um & lt);
+    // every entry of the list against the window of the one before it
+    const unsigned later = um & ~((2u << lane) - 1u);
+    float dn = __shfl_sync(0xffffffffu, d, later ? __ffs(later) - 1 : lane);
+    if (!later) dn = after;
+    const bool in = under && rk < kList;
+    const bool clear = !use_pen || dn >= __fadd_rn(d, two_w);
+    const bool flat = __all_sync(0xffffffffu, !in || clear);
+    const uint32_t tag = 0x00010000u | list_tag(c, epoch);
+    // (every lane stores, the same instructions: no branch to come together from)
+    auto entry = [&](unsigned long long* to, uint32_t ranks, uint32_t mat, int pos, bool clear) {
+      *reinterpret_cast<volatile unsigned long long*>(to) =
+          (unsigned long long)(tag | ((uint32_t)pos << 25) | (clear ? kClear : 0u) | mat) << 32 |
+          __funnelshift_r(ranks, ranks, 2);
+    };
+    if (cnt < kList) {
+      const bool none = lane < kList && lane >= cnt;
+      entry(none ? &Q.ent[slot][lane] : &Q.spare[0], 0xFFFFFFFFu, (uint32_t)p, lane & 7, true);
+      entry(none ? &Q.fin[slot][lane] : &Q.spare[0], 0xFFFFFFFFu, (uint32_t)p, lane & 7, true);
+    }
+    // the first form at once when the entries that mostly win are clear
+    const bool early = __all_sync(0xffffffffu, !under || rk >= kEarly || clear);
+    if (early) entry(in ? &Q.ent[slot][rk] : &Q.spare[0], 0x11111111u * (uint32_t)min(rk, 15), m & 0xFFFFu, rk & 7, clear);
+    // the list, for this cell's table and the next one's
+    const int put = in ? rk : kList;
+    Q.sel[slot][put] = make_float4(la.x, la.y, la.z, __uint_as_float(m));
+    Q.dw[r][put] = make_float2(d, wu);
+    __syncwarp();
+    st_release_cta(&Q.seq[slot], (uint32_t)(c + 1));
+    if (!flat) {
+      const float beyond =  // the distance of the first entry after the list
+          cnt > kList
+              ? __uint_as_float(__reduce_min_sync(0xffffffffu, under && rk == kList ? __float_as_uint(d) : 0xFFFFFFFFu))
+              : after;
+      // lane (i, j0) ranks entry i for previous entries j0 and j0 + 4
+      const bool absent = i >= cnt;
+      const float4 ei = Q.sel[slot][absent ? 0 : i];
+      const float2 di = Q.dw[r][absent ? 0 : i];
+      const float up_pen = __fadd_rn(0.0f, di.y);
+      float wa = 0.0f, wb = 0.0f;
+      if (x > 0) {
+        const int prev = (c - 1) & (kLists - 1);
+        if (!wait([&] { return ld_acquire_cta(&Q.seq[prev]) == (uint32_t)c; })) return;
+        const float4 ea = Q.sel[prev][j0], eb = Q.sel[prev][j0 + 4];  // stale beyond its length: never looked up
+        const float2 w = weight_of_sq2(sq_dist(ei.x, ei.y, ei.z, ea.x, ea.y, ea.z), sq_dist(ei.x, ei.y, ei.z, eb.x, eb.y, eb.z));
+        wa = w.x;
+        wb = w.y;
+      }
+      const float sa = absent ? inf : __fadd_rn(di.x, __fmul_rn(__fadd_rn(up_pen, wa), weight));
+      const float sb = absent ? inf : __fadd_rn(di.x, __fmul_rn(__fadd_rn(up_pen, wb), weight));
+      uint32_t ra = 0u, rb = 0u;
+#pragma unroll
+      for (int o = 1; o < kList; ++o) {
+        const int q = (i + o) & 7;
+        const float va = __shfl_sync(0xffffffffu, sa, (lane & 24) | q), vb = __shfl_sync(0xffffffffu, sb, (lane & 24) | q);
+        ra += va < sa || (va == sa && q < i) ? 1u : 0u;
+        rb += vb < sb || (vb == sb && q < i) ? 1u : 0u;
+      }
+      if (!(sa <= beyond)) ra = kRankOpen;
+      if (!(sb <= beyond)) rb = kRankOpen;
+      uint32_t ranks = (ra << (28 - 4 * j0)) | (rb << (12 - 4 * j0));
+      ranks |= __shfl_xor_sync(0xffffffffu, ranks, 8);
+      ranks |= __shfl_xor_sync(0xffffffffu, ranks, 16);
+      // (the four lanes of an entry hold the same word)
+      entry(absent ? &Q.spare[0] : early ? &Q.fin[slot][i] : &Q.ent[slot][i], ranks, __float_as_uint(ei.w) & 0xFFFFu, i, true);
+    }
+    __syncwarp();
+    st_release_cta(&Q.done[slot], (uint32_t)(c + 1));
+    // the next cell's record
+    const int next = c + kRefiners;
+    have = next < n && published(next);
+    if (have) load_record(next);
+    x += kRefiners;
+    while (x >= gw) x -= gw;
+  }
+}
+
+template <bool kLabSmem, bool kRing>
+__global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThreads, 1)
     greedy_pair_kernel(const float4* __restrict__ pal, int p, const GreedyJob* __restrict__ jobs, uint32_t* err,
                        uint32_t walk_polls, uint32_t withhold) {
   extern __shared__ __align__(128) uint8_t smem[];
   const GreedyJob J = jobs[blockIdx.x / (1 + kScoutCtas)];
   const uint32_t rank = cluster_ctarank();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp index through a shuffle: the compiler then knows each warp's path
+  // as converged (without, every warp collective of the walker's loop comes with
+  // a convergence step: 138 against 86 cycles a cell in a copy of the loop)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int gw = J.gw, gh = J.gh, k = J.k, n = gw * gh;
   const int R = ring_size(gw);
   const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
   if (rank == 0) {
-    for (int i = threadIdx.x; i < p; i += blockDim.x) {
-      L.usage[i] = 0;
-      if (kLabSmem) L.lab[i] = pal[i];
+    for (int i = threadIdx.x; i <= p; i += blockDim.x) {
+      L.usage[i] = i < p ? 0u : 0x7FFFFFFFu;  // absent entries have no room under any cap
+      if (kLabSmem && i < p) L.lab[i] = pal[i];
     }
+    for (int i = threadIdx.x; i < kLists * kList; i += blockDim.x)  // lists of no cell, their entries absent
+      (&L.lists->ent[0][0])[i] = (unsigned long long)(kTagCell | (uint32_t)p) << 32;
+    if (threadIdx.x < kLists) L.lists->seq[threadIdx.x] = L.lists->done[threadIdx.x] = 0;
     for (int i = threadIdx.x; i < R; i += blockDim.x) L.seq[i] = 0;
     if (kRing)
       for (int i = threadIdx.x; i < cell_ring_size(gw); i += blockDim.x) L.ring[i] = kNoCell;
@@ -570,15 +908,24 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWar
       for (int i = threadIdx.x; i < n; i += blockDim.x) L.grid16[i] = kUnplaced;
     if (threadIdx.x < 4) L.ctrl[threadIdx.x] = 0;
   }
-  cluster_sync_all();  // the walker CTA's state exists before any scout reads it
+  if (rank > 0) {
+    const ScoutLayout F = scout_layout(smem, p);
+    for (int i = threadIdx.x; i < p; i += blockDim.x) F.usage[i] = 0;
+    if (threadIdx.x < 4) F.ctl[threadIdx.x] = 0;
+  }
+  cluster_sync_all();  // the walker CTA's state exists before any follower reads it
 
   if (rank >= 1) {
     // ---- the scouts, then (CTA 1) the final cost of the walk
-    ScoutStage* stage = reinterpret_cast<ScoutStage*>(smem);
-    float* terms = reinterpret_cast<float*>(smem + (size_t)kWarps * sizeof(ScoutStage));
-    static_assert(kScoutCtas * kWarps == kScouts, "64 scouts");
-    bool ok = scout_cells<kRing, kScoutCtas == 4 ? kScoutLead : kScoutLeadBatch>((int)(rank - 1) * kWarps + warp, J, pal, p, smem, stage[warp], R, err,
-                                       withhold != 0u);
+    const ScoutLayout F = scout_layout(smem, p);
+    float* terms = F.terms;
+    constexpr int kPer = kScoutWarpsMax - 1;  // scouts in this CTA; its last warp follows the walk
+    bool ok = true;
+    if (warp < kPer)
+      ok = scout_cells<kRing, kScoutLead, kScoutCtas * kPer>(
+          (int)(rank - 1) * kPer + warp, J, pal, p, smem, F.stage[warp], R, err, withhold != 0u);
+    else
+      follow_walk<kRing>(J, p, smem, R, err);
     if (rank > 1) {
       cluster_sync_all();
       return;
@@ -631,7 +978,7 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWar
         }
         __syncthreads();
         if (threadIdx.x == 0)
-          for (int i = 0; i < 2 * m; ++i) total = __fadd_rn(total, terms[i]);
+          for (int i = 0; i < 2 * m; ++i) total = __fadd_rn(total, terms[i]);  // (the loads run ahead)
         __syncthreads();
       }
       if (threadIdx.x == 0 && J.total_cost) *J.total_cost = total;
@@ -694,21 +1041,19 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWar
     return;
   }
   if (warp != 0) {
+    // ---- CTA 0, the refiners (not on the walker's scheduler)
+    const int r = warp - warp / 4 - 2;
+    if ((warp & 3) != 0 && r >= 0 && r < kRefiners) refine_cells<kLabSmem, kRing>(r, J, pal, p, smem, R, err);
     cluster_sync_all();
     return;
   }
 
   // ---- CTA 0, warp 0: the walker
-  // Windows that are not clear are settled inside the common loop in the
-  // batch shape (dense palettes: a fifth of a batch's cells had one, each
-  // leaving the loop), and on the uncommon path in the five-CTA shape, whose
-  // loop the larger body slowed.
-  constexpr bool kInlineWindows = kScoutCtas == 2;
   uint32_t* ctrl = L.ctrl;
   CellRecord* rec = L.rec;
-  uint32_t* seq = L.seq;
   uint32_t* ring = L.ring;
   uint16_t* grid16 = L.grid16;
+  ListShared& Q = *L.lists;
   const int cmask = cell_ring_size(gw) - 1;
   // a placement: the 16-bit grid, or the ring word and the global grid
   auto place = [&](int cc, int tt) {
@@ -725,78 +1070,34 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWar
   const float weight = J.weight;
   auto lab = [=](int i) -> float4 { return kLabSmem ? s_lab[i] : __ldg(pal + i); };
   uint32_t epoch = 0;
-  int resets = 0, last = -1, x = 0, y = 0;
-  int ready_until = 0;  // records of cells [.., ready_until) are published
+  int resets = 0, last = -1, x = 0;
   bool aborted = false;
-  // Whether the record of cell c is published.  Records [0, ready_until) are
-  // known to be; a probe checks the next 32 (lane i acquires the sequence word
-  // of cell ready_until + i).  With `block` it waits (bounded).
-  auto ready = [&](int c, bool block) -> bool {
-    if (c < ready_until) return true;
-    uint32_t polls = 0;
-    for (;;) {
-      const int base = ready_until;
-      const int cc = base + lane;
-      const bool mine = cc >= n || ld_acquire_cluster(smem_u32(&seq[cc & (R - 1)])) == (uint32_t)(cc + 1);
-      const unsigned pending = __ballot_sync(0xffffffffu, !mine);
-      const int nready = pending ? __ffs(pending) - 1 : 32;
-      if (nready > 0) {
-        ready_until = min(n, base + nready);
-        __syncwarp();  // the acquiring lanes' view reaches every lane
-      }
-      if (c < ready_until) return true;
-      if (!block) return false;
-      if (++polls > walk_polls || ld_volatile_u32(&ctrl[kAbort])) {
-        aborted = true;
-        return false;
-      }
-    }
-  };
-  // The walk is a chain of dependent decisions, so its speed is the latency
-  // of one decision in one warp: every warp collective and every memory wait
-  // on the path from one cell's choice to the next counts in full.  Per cell,
-  // one warp minimum over the record's entries under the usage cap, the left
-  // neighbour's material removed, gives the reference's choice.  A record's
-  // counters are read before the previous commit; the only counter that
-  // commit changed is the left neighbour's, which is removed anyway -- except
-  // at a row start (no left neighbour), where that entry counts with its
-  // counter + 1.  Record reads are software-pipelined: the counters of cell
-  // c + 1 and the header of cell c + 2 are read first while cell c is
-  // decided, unconditionally (a record not yet published is read again once
-  // it is).  Everything uncommon (the full evaluation, windows that are not
-  // clear, late records and the probes for new ones) sits behind one branch.
-  // Placements go to the shared-memory grid, which the scouts poll; the grid
-  // reaches global memory once, after the walk.
-  struct Head {
-    uint32_t ep, kf, kr;
-  };
+  // A cell whose list does not settle it is decided from its record: the
+  // lowest key among the entries under the cap, not the left neighbour, is the
+  // reference's choice when its window is clear.
   struct Cur {
     uint32_t key, ti, ui;
     bool f;  // the key is the record's f entry (its epoch is the walk's)
   };
-  auto load_head = [&](int c) {
+  auto record_entry = [&](int c) {
+    (void)ld_acquire_cta(&Q.seq[c & (kLists - 1)]);  // its refiner saw the record published
     const CellRecord& Rc = rec[c & (R - 1)];
-    return Head{Rc.epoch, Rc.kf[lane], Rc.kr[lane]};
-  };
-  auto finish = [&](const Head& h) {
     Cur r;
-    r.f = h.ep == epoch;
-    r.key = r.f ? h.kf : h.kr;
+    r.f = Rc.epoch == epoch;
+    r.key = r.f ? Rc.kf[lane] : Rc.kr[lane];
     r.ti = r.key & 0xFFFFu;
     r.ui = (r.key != 0xFFFFFFFFu && r.ti < (uint32_t)p) ? usage[r.ti] : 0xFFFFFFFFu;
     return r;
   };
   // A cell (not a row start) whose first eligible f entry has later entries
-  // inside its penalty window, settled from the record when the palette's Lab
-  // is in global memory: the window's entries are the list's entries under the
-  // cap now, other than the left neighbour's material, with distance below
-  // d(first) + 2*weight (f_next >= that bound closes the window inside the
-  // list); each scores d + (w_up + w_left) * weight in full_cell's arithmetic
-  // and the lowest score, then the lowest position, wins -- full_cell's
-  // decision.  Commits it and returns the material; -1 when the window may
-  // reach past the list (then full_cell decides).  e0: the position of the
-  // first eligible entry (the loop's minimum).  Positions and materials come
-  // out of warp minimums over packed words (no bit scans or shuffles).
+  // inside its penalty window, settled from the record: the window's entries
+  // are the list's entries under the cap now, other than the left neighbour's
+  // material, with distance below d(first) + 2*weight (f_next >= that bound
+  // closes the window inside the list); each scores d + (w_up + w_left) *
+  // weight in full_cell's arithmetic and the lowest score, then the lowest
+  // position, wins -- full_cell's decision.  Commits it and returns the
+  // material; -1 when the window may reach past the list (then full_cell
+  // decides).  e0: the position of the first eligible entry.
   auto window_cell = [&](int cc, const Cur& cu, int left, bool has_up, int e0) -> int {
     const CellRecord& Rc = rec[cc & (R - 1)];
     const bool elig = cu.key != 0xFFFFFFFFu && cu.ui < max_usage && (int)cu.ti != left;
@@ -804,14 +1105,8 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWar
     const float b0 = __fadd_rn(Rc.wd[e0], __fmul_rn(2.0f, weight));
     if (!(Rc.f_next >= b0)) return -1;
     const bool in = elig && lane >= e0 && dl < b0;
-    // the left neighbour's Lab: its entry in the previous cell's list, else the palette
-    const CellRecord& Rp = rec[(cc - 1) & (R - 1)];
-    const uint32_t pk = Rp.kf[lane];
-    const uint32_t pl =
-        __reduce_min_sync(0xffffffffu, (pk != 0xFFFFFFFFu && (pk & 0xFFFFu) == (uint32_t)left) ? (uint32_t)lane : 32u);
-    const float4 lab_left = pl < 32u ? Rp.wl[pl] : lab(left);
     float pen = has_up ? Rc.wu[lane] : 0.0f;  // 0 + w_up, exactly
-    pen = __fadd_rn(pen, wgt(Rc.wl[lane], lab_left));
+    pen = __fadd_rn(pen, wgt(Rc.wl[lane], lab(left)));
     const uint32_t sb = in ? __float_as_uint(__fadd_rn(dl, __fmul_rn(pen, weight))) : 0xFFFFFFFFu;
     const uint32_t mn = __reduce_min_sync(0xffffffffu, sb);
     const bool wins = mn == 0xFFFFFFFFu ? lane == e0 : (in && sb == mn);
@@ -823,181 +1118,150 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __maxnreg__(65536 / (kWar
     }
     return tw;
   };
-  Cur cur{0xFFFFFFFFu, 0u, 0xFFFFFFFFu, false};
-  bool cur_fresh = true;  // cur's counters include the previous commit
-  Head h1{0u, 0xFFFFFFFFu, 0xFFFFFFFFu};
-  bool h1_ok = false;
-  if (n > 0 && ready(0, true)) {
-    cur = finish(load_head(0));
-    h1_ok = n > 1 && ready(1, false);
-    h1 = load_head(1 < n ? 1 : 0);
-  }
-  // The common case runs in a tight inner loop of its own; a cell that needs
-  // anything else leaves it, is finished below, and the inner loop resumes.
-  // Each entry's packed word (position << 27 | blocked << 26 | counter << 16 |
-  // material, ~0 unless present and under the cap) is formed when its
-  // counter arrives, with the counter as read (wb) and with one more (wp: the
-  // entry of a row start whose material the previous cell took, read before
-  // that commit).  The decision is then one warp minimum over the words with
-  // the left neighbour's material removed, and its commit is made by every
-  // lane (the same stores), so no lane waits on another before the next
-  // cell's counters are read.  The counter packs to 10 bits: an entry under
-  // the cap whose counter does not fit (caps above 1023) is marked as not
-  // clear, so a cell that would take it goes the uncommon way.
-  struct Words {
-    uint32_t ti, wb, wp;
+  // The walk is a chain of dependent decisions, so its speed is the latency of
+  // one decision in one warp.  Per cell that is a rotation and an OR (the ranks'
+  // column for the previous choice), one warp minimum, and the commit, made by
+  // every lane with the same stores so that no lane waits on another.  All else
+  // runs ahead: a list is read two cells early, unconditionally (one not there
+  // yet, or of another epoch, shows by its tag), its counters one cell early --
+  // the one commit in between is the left neighbour's, which the cell may not
+  // take -- and formed into the packed word beside the minimum of the cell
+  // before: rank << 28 | position << 25 | clear << 24 | counter + 1 << 16 | material;
+  // bits 23-27 are then the rotation that brings up the next column.  Counters pack to 7 bits: with caps
+  // beyond that (kWide) one of 127 or more is read again at its commit.
+  struct Entry {
+    uint32_t ranks, hi;
   };
-  auto words = [&](const Cur& r) -> Words {
-    const uint32_t base = ((r.key >> 17) << 27) | (((r.key >> 16) & 1u) << 26) | (r.key & 0xFFFFu);
-    const bool pres = r.key != 0xFFFFFFFFu;
-    Words o;
-    o.ti = r.ti;
-    o.wb = pres & (r.ui < max_usage) ? base | (min(r.ui, 1023u) << 16) | (r.ui < 1023u ? 0u : 1u << 26) : 0xFFFFFFFFu;
-    o.wp = pres & (r.ui + 1u < max_usage) ? base | (min(r.ui + 1u, 1023u) << 16) | (r.ui + 1u < 1023u ? 0u : 1u << 26)
-                                         : 0xFFFFFFFFu;
-    return o;
+  auto load_entry = [&](int c) {
+    const unsigned long long v = *reinterpret_cast<const volatile unsigned long long*>(&Q.ent[c & (kLists - 1)][lane & 7]);
+    return Entry{(uint32_t)v, (uint32_t)(v >> 32)};
   };
-  const float two_w = __fmul_rn(2.0f, weight);
-  int last_pos = -1;  // position of the previous cell's choice in its record's f list, -1 unknown
-  bool win_tried = false;
-  int c = 0;
-  while (c < n && !aborted) {
-    win_tried = false;
-    Head h2{};
-    bool h2_ok = false;
-    Cur nxt = cur;
-    uint32_t chosen = 0xFFFFFFFFu;
-    bool fast = false;
-    Words wc = words(cur);
-    for (;;) {
-      // (a) counters of cell c + 1, read before this cell's commit; header of
-      // cell c + 2 -- whether it is published is known from the last probe
-      // (probes happen on the uncommon path; waiting here, before this cell's
-      // commit, could wait on a scout that waits on this cell)
-      nxt = finish(h1);
-      h2_ok = c + 2 < ready_until;
-      h2 = load_head(c + 2);
-      // (b) this cell: the first entry under the cap that is not the left
-      // neighbour's material (at a row start, that material's counter + 1)
-      const bool same = wc.ti == (uint32_t)last;
-      const uint32_t w = !same ? wc.wb : (x != 0 ? 0xFFFFFFFFu : (cur_fresh ? wc.wb : wc.wp));
-      uint32_t b = __reduce_min_sync(0xffffffffu, w);
-      if (kInlineWindows && (b != 0xFFFFFFFFu) & ((b & (1u << 26)) != 0u) & (x != 0) & cur.f) {
-        // (c) a window that is not clear, settled here (window_cell's
-        // decision) when the record closes it; the left neighbour's Lab comes
-        // from the previous record's entry it was chosen as, else the palette
-        win_tried = true;
-        const CellRecord& Rc = rec[c & (R - 1)];
-        const int e0 = (int)(b >> 27);
-        const float b0 = __fadd_rn(Rc.wd[e0], two_w);
-        if (Rc.f_next >= b0) {
-          const float dl = Rc.wd[lane];
-          const bool in = (w != 0xFFFFFFFFu) & (lane >= e0) & (dl < b0);
-          const float4 lab_left = last_pos >= 0 ? rec[(c - 1) & (R - 1)].wl[last_pos] : lab(last);
-          const float pen = __fadd_rn(Rc.wu[lane], wgt(Rc.wl[lane], lab_left));  // 0 + w_up, then + w_left
-          const uint32_t sb = in ? __float_as_uint(__fadd_rn(dl, __fmul_rn(pen, weight))) : 0xFFFFFFFFu;
-          const uint32_t mn = __reduce_min_sync(0xffffffffu, sb);
-          const uint32_t wn = __reduce_min_sync(0xffffffffu, (in & (sb == mn)) ? w : 0xFFFFFFFFu);
-          const uint32_t pk = (mn == 0xFFFFFFFFu ? b : wn) & ~(1u << 26);
-          if (((pk >> 16) & 1023u) != 1023u) b = pk;  // a counter that fits its field
-        }
+  const uint32_t cap = lane < kList ? max_usage : 0u;  // lanes past the list never take part
+  // Decides cells from c on, not past `end` (the row's), the first one from
+  // lists and counters read afresh; b: the word of the choice before c.
+  // Returns the first cell left open.
+  auto fast_cells = [&](auto wide, int c, int end, uint32_t& b, Entry e0) -> int {
+    constexpr bool kWide = decltype(wide)::value;
+    uint32_t w, ranks;
+    auto form = [&](const Entry& e, uint32_t u, int cell) {
+      const uint32_t v = e.hi ^ list_tag(cell, epoch);
+      const bool there = (v & kTagMask) == 0u;
+      w = u < cap ? v + ((kWide ? min(u, 126u) : u) << 16) : 0xFFFFFFFFu;
+      w = there ? w : kNotThere;
+      ranks = there ? e.ranks : 0u;
+    };
+    // clear, and a rank below 8
+    auto settles = [](uint32_t best) { return ((best ^ kClear) & (0x80000000u | kClear)) == 0u; };
+    // the entry's word given the choice before: its rank's column, out if it is that material
+    auto choice = [&](uint32_t b) -> uint32_t {
+      const uint32_t word = w | (__funnelshift_l(ranks, ranks, b >> 23) & 0xF0000000u);
+      return ((w ^ b) & 0xFFFFu) == 0u ? 0xFFFFFFFFu : word;
+    };
+    for (uint32_t polls = 0;;) {
+      uint32_t stop = 0u;  // the word that stopped the run
+      const uint32_t u0 = usage[e0.hi & 0xFFFFu];
+      Entry e1 = load_entry(c + 1);
+      form(e0, u0, c);
+      uint32_t u1 = usage[e1.hi & 0xFFFFu];
+      bool ok = true;
+      while (c < end) {
+        const uint32_t word = choice(b);
+        const Entry e2 = load_entry(c + 2);
+        const uint32_t best = __reduce_min_sync(0xffffffffu, word);
+        form(e1, u1, c + 1);
+        stop = best;
+        ok = settles(best);
+        if (!ok) break;
+        uint32_t u = __byte_perm(best, 0u, 0x4442);
+        if (kWide && u == 127u) u = usage[best & 0xFFFFu] + 1u;
+        usage[best & 0xFFFFu] = u;
+        place(c, (int)(best & 0xFFFFu));
+        u1 = usage[e2.hi & 0xFFFFu];
+        b = best;
+        e1 = e2;
+        ++c;
       }
-      fast = (b != 0xFFFFFFFFu) & !(b & (1u << 26));
-      if (!fast || !h1_ok) {
-        // the record's key form for the uncommon path; a row start is redone there
-        chosen = b != 0xFFFFFFFFu ? (((b >> 27) << 17) | (((b >> 26) & 1u) << 16) | (b & 0xFFFFu)) : b;
-        fast = fast && x != 0;
+      // done; or cell c is open; or its list is not there, or its first entry
+      // not clear and the second form decides: a short wait for that
+      if (ok || stop >= kRankOpen << 28) return c;
+      if (stop == kNotThere) {
+        do {
+          if (++polls > 256u) return c;
+          e0 = load_entry(c);
+        } while (!__all_sync(0xffffffffu, ((e0.hi ^ list_tag(c, epoch)) & kTagMask) == 0u));
+      } else {
+        while (!__all_sync(0xffffffffu, ld_acquire_cta(&Q.done[c & (kLists - 1)]) == (uint32_t)(c + 1)))
+          if (++polls > 256u) return c;
+        const unsigned long long v = Q.fin[c & (kLists - 1)][lane & 7];
+        e0 = Entry{(uint32_t)v, (uint32_t)(v >> 32)};
+      }
+    }
+  };
+  bool known = true;         // b names the previous choice's position in its list
+  uint32_t b = kClear;
+  int c = 0;
+  while (c < n) {
+    // the list of cell c (bounded wait: its refiner waits for nothing the walker has yet to do)
+    Entry e = load_entry(c);
+    for (uint32_t polls = 0; !__all_sync(0xffffffffu, ((e.hi ^ list_tag(c, 0)) & kTagCell) == 0u);) {
+      if (++polls > walk_polls || __any_sync(0xffffffffu, ld_volatile_u32(&ctrl[kAbort]) != 0u)) {
+        aborted = true;
         break;
       }
-      const int t = (int)(b & 0xFFFFu);
-      usage[t] = ((b >> 16) & 1023u) + 1u;
-      place(c, t);
-      if (kInlineWindows) {
-        last_pos = cur.f ? (int)(b >> 27) : -1;
-        win_tried = false;
-      }
-      last = t;
-      cur = nxt;
-      wc = words(nxt);
-      cur_fresh = false;
-      h1 = h2;
-      h1_ok = h2_ok;
-      const bool wrap = x + 1 == gw;
-      x = wrap ? 0 : x + 1;
-      y += wrap ? 1 : 0;
-      if (++c == n) break;
+      e = load_entry(c);
     }
-    if (c == n) break;
-    // ---- the uncommon path for cell c
-    int t = (int)(chosen & 0xFFFFu);
-    if (fast) {
-      // only the next record was late
-      if (lane == (int)(chosen >> 17)) {
-        usage[cur.ti] = cur.ui + 1u;
+    if (aborted) break;
+    const bool fresh = __all_sync(0xffffffffu, ((e.hi ^ list_tag(c, epoch)) & kTagMask) == 0u);
+    if (fresh && (x == 0 || known)) {
+      const int c0 = c;
+      if (x == 0) b |= 0xFFFFu;  // no left neighbour
+      if (max_usage < 127u) c = fast_cells(std::false_type{}, c, c + gw - x, b, e);
+      else c = fast_cells(std::true_type{}, c, c + gw - x, b, e);
+      __syncwarp();
+      if (c > c0) {
+        last = (int)(b & 0xFFFFu);
+        known = true;
+        x += c - c0;
+        if (x == gw) x = 0;
+        continue;
+      }
+    }
+    // ---- cell c from its record, or in full
+    const bool row_start = x == 0;
+    const Cur cu = record_entry(c);
+    const uint32_t key = __reduce_min_sync(
+        0xffffffffu, cu.ui < max_usage && (row_start || (int)cu.ti != last) ? cu.key : 0xFFFFFFFFu);
+    int t = (int)(key & 0xFFFFu);
+    bool done = key != 0xFFFFFFFFu && !(key & 0x10000u);
+    if (done) {
+      if (lane == (int)(key >> 17)) {
+        usage[cu.ti] = cu.ui + 1u;
         place(c, t);
       }
-    } else {
-      const bool row_start = x == 0;
-      bool done = false;
-      if (row_start) {
-        // no left neighbour: the previous commit's counter counts
-        const uint32_t ui = cur.ui + ((!cur_fresh && cur.ti == (uint32_t)last && cur.key != 0xFFFFFFFFu) ? 1u : 0u);
-        const uint32_t b = __reduce_min_sync(0xffffffffu, ui < max_usage ? cur.key : 0xFFFFFFFFu);
-        if (b != 0xFFFFFFFFu && !(b & 0x10000u)) {
-          t = (int)(b & 0xFFFFu);
-          if (lane == (int)(b >> 17)) {
-            usage[cur.ti] = ui + 1u;
-            place(c, t);
-          }
-          done = true;
-        }
-      }
-      if (!done && !win_tried && !row_start && chosen != 0xFFFFFFFFu && (chosen & 0x10000u) &&
-          rec[c & (R - 1)].epoch == epoch) {
-        const int tw = window_cell(c, cur, last, y > 0, (int)(chosen >> 17));
-        if (tw >= 0) {
-          t = tw;
-          done = true;
-        }
-      }
-      if (!done) {
-        const int up = y == 0 ? -1 : kRing ? (int)(ring[(c - gw) & cmask] & 0xFFFFu) : (int)grid16[c - gw];
-        if (kLabSmem)
-          t = full_cell(lab, J.cand_idx + (size_t)c * k, J.cand_dist + (size_t)c * k, k, p, up,
-                        row_start ? -1 : last, usage, max_usage, weight, ctrl, epoch, resets, lane);
-        else
-          t = full_cell_rows(lab, J.cand_idx + (size_t)c * k, J.cand_dist + (size_t)c * k, k, p, up,
-                             row_start ? -1 : last, usage, max_usage, weight, ctrl, epoch, resets, lane);
-        if (lane == 0) place(c, t);
-      }
+    } else if (!row_start && key != 0xFFFFFFFFu && cu.f) {
+      const int tw = window_cell(c, cu, last, c >= gw, (int)(key >> 17));
+      done = tw >= 0;
+      if (done) t = tw;
+    }
+    if (!done) {
+      const int up = c < gw ? -1 : kRing ? (int)(ring[(c - gw) & cmask] & 0xFFFFu) : (int)grid16[c - gw];
+      const uint32_t* ci = J.cand_idx + (size_t)c * k;
+      const float* cd = J.cand_dist + (size_t)c * k;
+      if (kLabSmem)
+        t = full_cell(lab, ci, cd, k, p, up, row_start ? -1 : last, usage, max_usage, weight, ctrl, epoch, resets, lane,
+                      Q.reset_at, c);
+      else
+        t = full_cell_rows(lab, ci, cd, k, p, up, row_start ? -1 : last, usage, max_usage, weight, ctrl, epoch, resets, lane,
+                      Q.reset_at, c);
+      if (lane == 0) place(c, t);
     }
     __syncwarp();
-    bool nxt_fresh = false;
-    if (c + 1 < n) {
-      if (!h1_ok) {
-        h1_ok = ready(c + 1, true);
-        h1 = load_head(c + 1);
-      }
-      // the counters moved (a full evaluation), or the record came late: read afresh
-      nxt = finish(h1);
-      nxt_fresh = true;
-      // look ahead for the records of the coming cells (one probe covers 32)
-      if (ready_until < n && ready_until <= c + 32) (void)ready(ready_until, false);
-      if (!h2_ok && c + 2 < ready_until) {
-        h2_ok = true;
-        h2 = load_head(c + 2);
-      }
-    }
     last = t;
-    last_pos = -1;
-    cur = nxt;
-    cur_fresh = nxt_fresh;
-    h1 = h2;
-    h1_ok = h2_ok;
-    const bool wrap = x + 1 == gw;
-    x = wrap ? 0 : x + 1;
-    y += wrap ? 1 : 0;
+    const unsigned at = __ballot_sync(0xffffffffu, lane < kList && (e.hi & 0xFFFFu) == (uint32_t)t);
+    known = at != 0u;
+    b = kClear | (known ? (uint32_t)(__ffs(at) - 1) << 25 : 0u) | (uint32_t)t;
     ++c;
+    x = x + 1 == gw ? 0 : x + 1;
   }
   if (aborted) {
     if (lane == 0) {
@@ -1028,7 +1292,7 @@ size_t greedy_shared_bytes(int k, int gw, int p, bool lab_smem, bool usage_smem)
 }
 
 bool greedy_scouted_fits(int gw, int n, int p) {
-  constexpr size_t kMaxSmem = 220 * 1024;
+  constexpr size_t kMaxSmem = 227 * 1024 - 128;  // beside the kernel's static words
   // the largest ring any row width uses, the palette Lab outside shared memory
   return gw >= 8 && p <= 65535 &&
          (pair_smem_bytes(gw, n, p, false, false) <= kMaxSmem || pair_smem_bytes(gw, n, p, false, true) <= kMaxSmem);
@@ -1039,8 +1303,8 @@ int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_job
                   bool inject_timeout) {
   if (n_jobs <= 0) return MG_OK;
   if (k < 1 || k > 100) return fail(MG_ERR_ARG, "candidate count must be in 1..100");
-  constexpr size_t kMaxSmem = 220 * 1024;
-  static int configured_device = -1, sms = 0;
+  constexpr size_t kMaxSmem = 227 * 1024 - 128;  // beside the kernel's static words
+  static int configured_device = -1;
   int dev = 0;
   MG_CUDA(cudaGetDevice(&dev));
   if (configured_device != dev) {
@@ -1049,15 +1313,10 @@ int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_job
     MG_CUDA(cudaFuncSetAttribute(greedy_kernel<true, true>, a, m));
     MG_CUDA(cudaFuncSetAttribute(greedy_kernel<false, true>, a, m));
     MG_CUDA(cudaFuncSetAttribute(greedy_kernel<false, false>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<true, false, 4, 16>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<false, false, 4, 16>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<true, true, 4, 16>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<false, true, 4, 16>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<true, false, 2, 32>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<false, false, 2, 32>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<true, true, 2, 32>, a, m));
-    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<false, true, 2, 32>, a, m));
-    MG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<true, false>, a, m));
+    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<false, false>, a, m));
+    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<true, true>, a, m));
+    MG_CUDA(cudaFuncSetAttribute(greedy_pair_kernel<false, true>, a, m));
     configured_device = dev;
   }
   // The scouted walk: counters in shared memory, 16-bit palette indices, rows
@@ -1073,22 +1332,13 @@ int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_job
       const bool lab_smem = form == 0 || form == 2, ring = form >= 2;
       const size_t bytes = pair_smem_bytes(max_gw, max_cells, p, lab_smem, ring);
       const uint32_t polls = inject_timeout ? kInjectedWalkPolls : kWalkPolls, hold = inject_timeout ? 1u : 0u;
-      // five SMs a mosaic while every cluster finds room at once, else three
-      const bool wide = 5 * n_jobs <= sms;
-      auto go = [&](auto kernel, int ctas, int threads) {
-        kernel<<<(unsigned)(ctas * n_jobs), threads, bytes, stream>>>(pal, p, jobs_dev, err, polls, hold);
+      auto go = [&](auto kernel) {
+        kernel<<<(unsigned)((1 + kScoutCtas) * n_jobs), kThreads, bytes, stream>>>(pal, p, jobs_dev, err, polls, hold);
       };
-      if (wide) {
-        if (form == 0) go(greedy_pair_kernel<true, false, 4, 16>, 5, 512);
-        else if (form == 1) go(greedy_pair_kernel<false, false, 4, 16>, 5, 512);
-        else if (form == 2) go(greedy_pair_kernel<true, true, 4, 16>, 5, 512);
-        else go(greedy_pair_kernel<false, true, 4, 16>, 5, 512);
-      } else {
-        if (form == 0) go(greedy_pair_kernel<true, false, 2, 32>, 3, 1024);
-        else if (form == 1) go(greedy_pair_kernel<false, false, 2, 32>, 3, 1024);
-        else if (form == 2) go(greedy_pair_kernel<true, true, 2, 32>, 3, 1024);
-        else go(greedy_pair_kernel<false, true, 2, 32>, 3, 1024);
-      }
+      if (form == 0) go(greedy_pair_kernel<true, false>);
+      else if (form == 1) go(greedy_pair_kernel<false, false>);
+      else if (form == 2) go(greedy_pair_kernel<true, true>);
+      else go(greedy_pair_kernel<false, true>);
       g_launches += 1;
       MG_CUDA(cudaGetLastError());
       return MG_OK;
