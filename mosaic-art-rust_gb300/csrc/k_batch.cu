@@ -35,10 +35,9 @@ constexpr int kCellBaseSmem = 1024;  // mosaics whose first cells the cell kerne
 // cell indices into shared memory once, so finding a cell's mosaic is a
 // binary search on chip.
 template <int kWarps>
-__global__ void __launch_bounds__(32 * kWarps) batch_cells_kernel(const BatchMosaic* __restrict__ mos, int nm,
-                                                                  int total_cells, const LabConsts* __restrict__ C,
-                                                                  float4* __restrict__ lab_out,
-                                                                  uchar4* __restrict__ rgb_out) {
+__global__ void __launch_bounds__(32 * kWarps, kLabThreadsPerSm / (32 * kWarps))
+    batch_cells_kernel(const BatchMosaic* __restrict__ mos, int nm, int total_cells, const LabConsts* __restrict__ C,
+                       float4* __restrict__ lab_out, uchar4* __restrict__ rgb_out) {
   __shared__ float s_lut[256];
   __shared__ int s_base[kCellBaseSmem];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = C->lut[i];
@@ -73,13 +72,12 @@ __global__ void __launch_bounds__(32 * kWarps) batch_cells_kernel(const BatchMos
     const int cy = local / M.gw, cx = local - cy * M.gw;
     const uint8_t* base = M.target + (int64_t)cy * M.ch * M.stride + 3ll * cx * M.cw;
     LabAcc acc;
-    reduce_rows<true>(base, M.cw, M.stride, 0, M.ch, lane, s_lut, K, acc);
-    const LabSums t = warp_sums<true>(acc);
+    reduce_rows<true>(base, M.cw, M.stride, 0, M.ch, lane, 32, s_lut, K, acc);
+    const LabSums t = lane_sums<true>(acc, 32);
     if (lane == 0) {
       const long long npx = (long long)M.cw * M.ch;
-      const unsigned long long n = (unsigned long long)npx;
       lab_out[cell] = make_float4(lab_mean(t.L, npx), lab_mean(t.A, npx), lab_mean(t.B, npx), 0.0f);
-      rgb_out[cell] = make_uchar4((unsigned char)(t.R / n), (unsigned char)(t.G / n), (unsigned char)(t.Bc / n), 0);
+      rgb_out[cell] = rgb_mean(t, npx);
     }
   }
 }

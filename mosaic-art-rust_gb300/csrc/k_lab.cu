@@ -6,10 +6,11 @@
 // truncating division), main.rs:495-496 / 537-541 (cells of w/gw x h/gh at
 // (x*cw, y*ch), remainder ignored).
 //
-// Design: one warp per (region, chunk of rows); the per-pixel work is
-// lab_reduce.cuh (packed FP32x2 Lab of pixel pairs from 48-byte loads,
+// Design: one team of threads per (region, chunk of rows), a part of a warp up to
+// a CTA by the number and size of the regions; the per-pixel work is
+// lab_reduce.cuh (packed FP32x2 Lab of pixel pairs from 24-byte loads,
 // fixed-point sums).  A region that fits one unit (a target cell) is reduced
-// and divided by its warp; larger ones (materials) add each chunk's sums to
+// and divided by its team; larger ones (materials) add each chunk's sums to
 // the region's with 64-bit atomics and a second tiny kernel divides.  Integer
 // sums are exact, so the result does not depend on the split.
 #include <cmath>
@@ -66,29 +67,34 @@ constexpr int kStatThreads = 256;
 constexpr int kStatWarps = kStatThreads / 32;
 constexpr int64_t kUnitPx = 4096;  // pixels per warp unit when a region is split into row chunks
 
-// One warp per unit = (region, chunk of its rows).  With one chunk per region
-// the unit's warp writes the region's means itself; with several, it adds its
-// sums to the region's (zeroed) RegionSums with six 64-bit atomics and
-// region_finalize_kernel divides.  The CTA loads the transfer table once and
-// its warps take units round robin.
+// One team of threads per unit = (region, chunk of its rows): 8, 16 or 32 lanes
+// of a warp, or 2, 4 or 8 warps of the CTA that add their sums up in shared
+// memory (team_size).  With one chunk per region the unit's team writes the
+// region's means itself; with several, it adds its sums to the region's (zeroed)
+// RegionSums with six 64-bit atomics and region_finalize_kernel divides.  The
+// CTA loads the transfer table once and its teams take units round robin.
 template <bool kCells, bool kLab>
-__global__ void __launch_bounds__(kStatThreads) region_stats_kernel(const uint8_t* __restrict__ base, CellGeom geom,
-                                                                    const Region* __restrict__ regions, int n_regions,
-                                                                    int chunks, RegionSums* __restrict__ sums,
-                                                                    float4* __restrict__ out_lab,
-                                                                    uchar4* __restrict__ out_rgb) {
+__global__ void __launch_bounds__(kStatThreads, kLabThreadsPerSm / kStatThreads)
+    region_stats_kernel(const uint8_t* __restrict__ base, CellGeom geom, const Region* __restrict__ regions,
+                        int n_regions, int chunks, int team, RegionSums* __restrict__ sums,
+                        float4* __restrict__ out_lab, uchar4* __restrict__ out_rgb) {
   __shared__ float s_lut[256];
+  __shared__ LabSums s_part[kStatWarps];
   if (kLab) {
     for (int i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = c_lab.lut[i];
     __syncthreads();
   }
   const LabK K = make_lab_k(c_lab.ms, c_lab.eps, c_lab.k1, c_lab.k2);
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & (team - 1), slot = threadIdx.x >> (31 - __clz(team)), per = kStatThreads >> (31 - __clz(team));
   const int64_t units = (int64_t)n_regions * chunks;
-  for (int64_t u = (int64_t)blockIdx.x * kStatWarps + (threadIdx.x >> 5); u < units;
-       u += (int64_t)gridDim.x * kStatWarps) {
-    const int r = (int)(u / chunks);
-    const int chunk = (int)(u - (int64_t)r * chunks);
+  for (int64_t u0 = (int64_t)blockIdx.x * per; u0 < units; u0 += (int64_t)gridDim.x * per) {
+    const int64_t u = u0 + slot;
+    const bool have = u < units;
+    int r = have ? (int)u : 0, chunk = 0;
+    if (chunks > 1 && have) {
+      r = (int)(u / chunks);
+      chunk = (int)(u - (int64_t)r * chunks);
+    }
     int64_t off, stride;
     int w, h;
     if (kCells) {
@@ -104,18 +110,36 @@ __global__ void __launch_bounds__(kStatThreads) region_stats_kernel(const uint8_
       h = reg.h;
       stride = reg.stride;
     }
-    const int y0 = (int)((int64_t)chunk * h / chunks), y1 = (int)((int64_t)(chunk + 1) * h / chunks);
+    int y0 = 0, y1 = h;
+    if (chunks > 1) {
+      y0 = (int)((int64_t)chunk * h / chunks);
+      y1 = (int)((int64_t)(chunk + 1) * h / chunks);
+    }
     LabAcc acc;
-    reduce_rows<kLab>(base + off, w, stride, y0, y1, lane, s_lut, K, acc);
-    const LabSums t = warp_sums<kLab>(acc);
-    if (lane == 0) {
+    if (have) reduce_rows<kLab>(base + off, w, stride, y0, y1, lane, team, s_lut, K, acc);
+    LabSums t = lane_sums<kLab>(acc, min(team, 32));
+    if (team > 32) {
+      if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = t;
+      __syncthreads();
+      if (lane == 0)
+        for (int i = 1; i < team / 32; ++i) {
+          const LabSums o = s_part[(threadIdx.x >> 5) + i];
+          t.L += o.L;
+          t.A += o.A;
+          t.B += o.B;
+          t.R += o.R;
+          t.G += o.G;
+          t.Bc += o.Bc;
+        }
+      __syncthreads();
+    }
+    if (have && lane == 0) {
       if (chunks == 1) {
         const long long npx = (long long)w * h;
         if (kLab && out_lab)
           out_lab[r] = make_float4(lab_mean(t.L, npx), lab_mean(t.A, npx), lab_mean(t.B, npx), 0.0f);
         if (out_rgb) {
-          const unsigned long long n = (unsigned long long)npx;
-          out_rgb[r] = make_uchar4((unsigned char)(t.R / n), (unsigned char)(t.G / n), (unsigned char)(t.Bc / n), 0);
+          out_rgb[r] = rgb_mean(t, npx);
         }
       } else {
         if (kLab) {
@@ -129,6 +153,28 @@ __global__ void __launch_bounds__(kStatThreads) region_stats_kernel(const uint8_
       }
     }
   }
+}
+
+// Threads per unit.  A team that is large for its unit wastes lanes in its last
+// step and on the sums; one that is small leaves schedulers idle where units are
+// few, and a lane's steps are a chain.  In cycles of a scheduler, for a step of
+// four pixels: 320 of its FMA pipe or 600 on its own; 250 for the rest of a
+// unit, and 600 more for the CTA's barriers.  Measured as whole calls, a warp a
+// cell -> this rule: 8 x 8 cells of 64 x 64 pixels 21 -> 8 us, 20 x 14 of 50 x 50
+// 23 -> 10, 161 x 78 of 4 x 4 23 -> 8.5, 160 x 90 of 24 x 24 41 -> 35.
+int team_size(int64_t units, int64_t unit_px, int sms) {
+  int best = 32;
+  double best_cost = 0.0;
+  for (int team = 8; team <= kStatThreads; team *= 2) {
+    const double warps = (double)units * team / (32.0 * 4.0 * sms);  // per scheduler
+    const double steps = (double)((unit_px / 4 + team - 1) / team);
+    const double cost = warps * (320.0 * steps + (team > 32 ? 850.0 : 250.0)) + 600.0 * steps;
+    if (team == 8 || cost < best_cost) {
+      best = team;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 template <bool kCells>
@@ -195,30 +241,31 @@ int launch_region_stats(const uint8_t* base, const CellGeom* geom, const Region*
                         int64_t max_region_px, float4* out_lab, uchar4* out_rgb, RegionSums* scratch, int want_lab,
                         cudaStream_t stream) {
   if (n_regions <= 0) return MG_OK;
+  int dev = 0, sms = 0;
+  MG_CUDA(cudaGetDevice(&dev));
+  MG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   // Regions above 2 units split into row chunks of about kUnitPx pixels, so
   // that a few large materials still spread over the GPU; smaller ones (target
-  // cells) are one warp each and need no scratch.
+  // cells) are one unit each and need no scratch.
   const int chunks = (int)std::min<int64_t>(64, std::max<int64_t>(1, max_region_px / kUnitPx));
   const int64_t units = (int64_t)n_regions * chunks;
   if (units > (1ll << 40)) return fail(MG_ERR_ARG, "too many regions");
   if (chunks > 1) MG_CUDA(cudaMemsetAsync(scratch, 0, sizeof(RegionSums) * (size_t)n_regions, stream));
-  int dev = 0, sms = 0;
-  MG_CUDA(cudaGetDevice(&dev));
-  MG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((units + kStatWarps - 1) / kStatWarps,
-                                                                         (int64_t)sms * 16));
+  const int team = team_size(units, max_region_px / chunks, sms);
+  const int per = kStatThreads / team;
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((units + per - 1) / per, (int64_t)sms * 16));
   CellGeom g{};
   if (geom) g = *geom;
   float4* lab = want_lab ? out_lab : nullptr;
   if (geom) {
-    if (want_lab) region_stats_kernel<true, true><<<grid, kStatThreads, 0, stream>>>(base, g, nullptr, n_regions, chunks, scratch, lab, out_rgb);
-    else region_stats_kernel<true, false><<<grid, kStatThreads, 0, stream>>>(base, g, nullptr, n_regions, chunks, scratch, lab, out_rgb);
+    if (want_lab) region_stats_kernel<true, true><<<grid, kStatThreads, 0, stream>>>(base, g, nullptr, n_regions, chunks, team, scratch, lab, out_rgb);
+    else region_stats_kernel<true, false><<<grid, kStatThreads, 0, stream>>>(base, g, nullptr, n_regions, chunks, team, scratch, lab, out_rgb);
     if (chunks > 1)
       region_finalize_kernel<true><<<(n_regions + 255) / 256, 256, 0, stream>>>(g, nullptr, n_regions, scratch, lab,
                                                                                out_rgb);
   } else {
-    if (want_lab) region_stats_kernel<false, true><<<grid, kStatThreads, 0, stream>>>(base, g, regions, n_regions, chunks, scratch, lab, out_rgb);
-    else region_stats_kernel<false, false><<<grid, kStatThreads, 0, stream>>>(base, g, regions, n_regions, chunks, scratch, lab, out_rgb);
+    if (want_lab) region_stats_kernel<false, true><<<grid, kStatThreads, 0, stream>>>(base, g, regions, n_regions, chunks, team, scratch, lab, out_rgb);
+    else region_stats_kernel<false, false><<<grid, kStatThreads, 0, stream>>>(base, g, regions, n_regions, chunks, team, scratch, lab, out_rgb);
     if (chunks > 1)
       region_finalize_kernel<false><<<(n_regions + 255) / 256, 256, 0, stream>>>(g, regions, n_regions, scratch, lab,
                                                                                 out_rgb);

@@ -1,5 +1,5 @@
 // lab_reduce.cuh -- per-pixel Lab and mean-RGB sums over rows of an RGB8
-// region, one warp at a time.  Shared by the region kernel (k_lab.cu: target
+// region, one team of threads at a time.  Shared by the region kernel (k_lab.cu: target
 // cells, materials, thumbnails) and the batch kernel (k_batch.cu: the cells
 // of many targets).
 //
@@ -7,17 +7,24 @@
 // summed, divided by the pixel count) and main.rs:687-708
 // calculate_average_rgb (integer sums).
 //
-// The reduction is issue-bound (three cube roots per pixel), so the design
-// minimises issued instructions per pixel:
+// What bounds it: three cube roots a pixel, that is 65 packed FP32
+// instructions and six 32-bit multiply-highs a pixel pair, 157 cycles of a
+// scheduler's FMA pipe (two a packed instruction, four a multiply-high); the
+// 25 MB of a 3840x2160 target take 4 us of them at the copy rate.  So:
 //   * pixels are converted two at a time in packed FP32x2 arithmetic
 //     (__ffma2_rn / __fmul2_rn / __fadd2_rn, each component rounded exactly
 //     as the scalar op), one pixel per component, so the result is
-//     mg_math.h's lab_pixel_q bit for bit;
-//   * a lane loads a group of 16, 8 or 4 pixels per step as three 16-, 8- or
-//     4-byte vectors (48, 24 or 12 bytes), the widest the row's alignment and
-//     width allow; other rows go pixel pair by pixel pair;
-//   * quantised Lab is summed in 32-bit registers within a group (at most 16
-//     pixels of |value| < 109 * 2^20) and folded into 64-bit sums once per
+//     mg_math.h's lab_pixel_q bit for bit: the pipe's time is that of scalar
+//     instructions, the issue slots are half;
+//   * the chain of a cube root is 16 dependent instructions, so the pipe is
+//     filled by warps: 80 registers a thread at most, 24 warps an SM (kLabThreadsPerSm)
+//     (at the compiler's own 97 to 159 registers, 8 to 16 warps: 45 us
+//     against 31 for 80x60 cells of 3840x2160, and 90 against 45 where the
+//     rows' alignment forces pixel pairs; 64 registers spill);
+//   * a lane loads a group of 8 or 4 pixels per step as three 8- or 4-byte
+//     vectors, one step ahead of its use (33 us without);
+//   * quantised Lab is summed in 32-bit registers within a group (at most 8
+//     pixels of |value| < 128 * 2^20) and folded into 64-bit sums once per
 //     group;
 //   * the sRGB transfer table sits in shared memory (one load per channel).
 // Integer sums are exact, so the result does not depend on how pixels are
@@ -26,6 +33,10 @@
 #include "mg_internal.h"
 
 namespace mg {
+
+// Threads an SM holds of the kernels that run this reduction: the second
+// argument of their launch bounds is kLabThreadsPerSm / threads per block.
+constexpr int kLabThreadsPerSm = 768;
 
 // The conversion constants, held per thread as packed pairs.
 struct LabK {
@@ -131,14 +142,7 @@ struct GroupSum {
 
 template <int kG>
 __device__ __forceinline__ void load_group(const uint8_t* p, uint32_t (&w)[3 * kG / 4]) {
-  if constexpr (kG == 16) {
-    const uint4* v = reinterpret_cast<const uint4*>(p);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const uint4 a = v[i];
-      w[4 * i] = a.x; w[4 * i + 1] = a.y; w[4 * i + 2] = a.z; w[4 * i + 3] = a.w;
-    }
-  } else if constexpr (kG == 8) {
+  if constexpr (kG == 8) {
     const uint2* v = reinterpret_cast<const uint2*>(p);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -153,33 +157,37 @@ __device__ __forceinline__ void load_group(const uint8_t* p, uint32_t (&w)[3 * k
 }
 
 // Rows [y0, y1) of a region w pixels wide, in groups of kG pixels (w a
-// multiple of kG; img and stride multiples of kG bytes).  Lane l takes groups
-// l, l + 32, ... in row-major order.
+// multiple of kG; img and stride multiples of kG bytes).  Lane l of the team
+// takes groups l, l + team, ... in row-major order, each loaded a step before it is used.
 template <int kG, bool kLab>
 __device__ __forceinline__ void rows_groups(const uint8_t* __restrict__ img, int w, int64_t stride, int y0, int y1,
-                                            int lane, const float* lut, const LabK& K, LabAcc& acc) {
+                                            int lane, int team, const float* lut, const LabK& K, LabAcc& acc) {
   const int gpr = w / kG;
   const int ng = (y1 - y0) * gpr;
   int gx = lane % gpr, y = y0 + lane / gpr;
-  const int dgx = 32 % gpr, dgy = 32 / gpr;
-  for (int q = lane; q < ng; q += 32) {
-    uint32_t wv[3 * kG / 4];
-    load_group<kG>(img + (int64_t)y * stride + 3 * kG * gx, wv);
-    int sL = 0, sA = 0, sB = 0;
-    unsigned sR = 0, sG = 0, sBc = 0;
-    GroupSum<kG, kLab>::run(wv, lut, K, sL, sA, sB, sR, sG, sBc);
-    acc.L += sL;
-    acc.A += sA;
-    acc.B += sB;
-    acc.R += sR;
-    acc.G += sG;
-    acc.Bc += sBc;
+  const int dgx = team % gpr, dgy = team / gpr;
+  uint32_t cur[3 * kG / 4];
+  if (lane < ng) load_group<kG>(img + (int64_t)y * stride + 3 * kG * gx, cur);
+  for (int q = lane; q < ng; q += team) {
+    uint32_t next[3 * kG / 4] = {};
     gx += dgx;
     y += dgy;
     if (gx >= gpr) {
       gx -= gpr;
       ++y;
     }
+    if (q + team < ng) load_group<kG>(img + (int64_t)y * stride + 3 * kG * gx, next);
+    int sL = 0, sA = 0, sB = 0;
+    unsigned sR = 0, sG = 0, sBc = 0;
+    GroupSum<kG, kLab>::run(cur, lut, K, sL, sA, sB, sR, sG, sBc);
+    acc.L += sL;
+    acc.A += sA;
+    acc.B += sB;
+    acc.R += sR;
+    acc.G += sG;
+    acc.Bc += sBc;
+#pragma unroll
+    for (int i = 0; i < 3 * kG / 4; ++i) cur[i] = next[i];
   }
 }
 
@@ -187,10 +195,10 @@ __device__ __forceinline__ void rows_groups(const uint8_t* __restrict__ img, int
 // odd width ends in a pair whose second pixel repeats the first and counts 0.
 template <bool kLab>
 __device__ __forceinline__ void rows_pairs(const uint8_t* __restrict__ img, int w, int64_t stride, int y0, int y1,
-                                           int lane, const float* lut, const LabK& K, LabAcc& acc) {
+                                           int lane, int team, const float* lut, const LabK& K, LabAcc& acc) {
   const int ppr = (w + 1) >> 1;
   const int np = (y1 - y0) * ppr;
-  for (int q = lane; q < np; q += 32) {
+  for (int q = lane; q < np; q += team) {
     const int row = q / ppr;
     const int x = 2 * (q - row * ppr);
     const uint8_t* p = img + (int64_t)(y0 + row) * stride + 3 * x;
@@ -210,28 +218,36 @@ __device__ __forceinline__ void rows_pairs(const uint8_t* __restrict__ img, int 
   }
 }
 
-// The lane's share of rows [y0, y1) of a region, by the widest group form the
-// geometry allows (warp-uniform: every lane sees the same region).
+// The share of rows [y0, y1) of a region of lane `lane` of a team of threads
+// (every lane sees the same region).  Rows that allow groups of 8 take those of 4 where
+// the team's last step is so empty that the smaller step wins: a step
+// costs about 17 units for 8 pixels and 9 for 4 (cells of 48x36: 31 us for
+// 80x60 of them in groups of 8, 33 in groups of 4; cells of 24x24: 41 and 37
+// for 160x90).
 template <bool kLab>
 __device__ __forceinline__ void reduce_rows(const uint8_t* img, int w, int64_t stride, int y0, int y1, int lane,
-                                            const float* lut, const LabK& K, LabAcc& acc) {
+                                            int team, const float* lut, const LabK& K, LabAcc& acc) {
   const uint64_t align = (uint64_t)(uintptr_t)img | (uint64_t)stride;
-  if ((w & 15) == 0 && (align & 15) == 0) rows_groups<16, kLab>(img, w, stride, y0, y1, lane, lut, K, acc);
-  else if ((w & 7) == 0 && (align & 7) == 0) rows_groups<8, kLab>(img, w, stride, y0, y1, lane, lut, K, acc);
-  else if ((w & 3) == 0 && (align & 3) == 0) rows_groups<4, kLab>(img, w, stride, y0, y1, lane, lut, K, acc);
-  else rows_pairs<kLab>(img, w, stride, y0, y1, lane, lut, K, acc);
+  bool by8 = (w & 7) == 0 && (align & 7) == 0;
+  if (by8) {
+    const int n8 = (y1 - y0) * (w >> 3);
+    by8 = 17 * ((n8 + team - 1) / team) <= 9 * ((2 * n8 + team - 1) / team);
+  }
+  if (by8) rows_groups<8, kLab>(img, w, stride, y0, y1, lane, team, lut, K, acc);
+  else if ((w & 3) == 0 && (align & 3) == 0) rows_groups<4, kLab>(img, w, stride, y0, y1, lane, team, lut, K, acc);
+  else rows_pairs<kLab>(img, w, stride, y0, y1, lane, team, lut, K, acc);
 }
 
-// Sums of the whole warp, in every lane (RGB widened to 64 bits).
+// Sums of each `width` lanes (a power of two) of the warp, in every one of them
+// (RGB widened to 64 bits).
 struct LabSums {
   long long L, A, B;
   unsigned long long R, G, Bc;
 };
 template <bool kLab>
-__device__ __forceinline__ LabSums warp_sums(const LabAcc& a) {
+__device__ __forceinline__ LabSums lane_sums(const LabAcc& a, int width) {
   LabSums s{a.L, a.A, a.B, a.R, a.G, a.Bc};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = width >> 1; o > 0; o >>= 1) {
     if (kLab) {
       s.L += __shfl_xor_sync(0xffffffffu, s.L, o);
       s.A += __shfl_xor_sync(0xffffffffu, s.A, o);
@@ -242,6 +258,17 @@ __device__ __forceinline__ LabSums warp_sums(const LabAcc& a) {
     s.Bc += __shfl_xor_sync(0xffffffffu, s.Bc, o);
   }
   return s;
+}
+
+// Truncated means; 32-bit divisions where the sums fit.
+__device__ __forceinline__ uchar4 rgb_mean(const LabSums& s, long long npx) {
+  if (npx <= 0xFFFFFFFFll / 255) {
+    const uint32_t n = (uint32_t)npx;
+    return make_uchar4((unsigned char)((uint32_t)s.R / n), (unsigned char)((uint32_t)s.G / n),
+                       (unsigned char)((uint32_t)s.Bc / n), 0);
+  }
+  const unsigned long long n = (unsigned long long)npx;
+  return make_uchar4((unsigned char)(s.R / n), (unsigned char)(s.G / n), (unsigned char)(s.Bc / n), 0);
 }
 
 }  // namespace mg
