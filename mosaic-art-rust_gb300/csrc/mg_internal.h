@@ -4,7 +4,9 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <map>
 #include <string>
+#include <vector>
 
 #include "../../include/mosaic_gpu.h"
 #include "mg_math.h"
@@ -75,7 +77,8 @@ int launch_gather(const int64_t* src, int n, size_t bytes, uint8_t* dst, cudaStr
 
 // Lanczos3 thumbnails of regions at tw x th (k_resize.cu): ResizePlan::build
 // makes the weight tables of the regions' sizes on the host and uploads them
-// (once per palette or plan); launch_resize runs the two passes.
+// (once per palette or plan) and decides how the passes run; launch_resize runs
+// them.
 struct ResizeImage {
   int64_t offset, stride;
   int32_t w, h;
@@ -84,8 +87,16 @@ struct ResizeImage {
 struct ResizePlan {
   DevBuf tabs, images, inter;
   int n = 0, tw = 0, th = 0, max_h = 0;
+  // both passes in one kernel: the CTAs of an image, and their shared memory in words
+  bool fused = false;
+  int bands = 1, hw_words = 0, vw_words = 0, src_words = 0, inter_pitch = 0;
   int build(const Region* regions, int n_images, int tw, int th, cudaStream_t s);
   void release();
+
+ private:
+  int build_images(const Region* regions, std::vector<int32_t>& t, std::map<int, int>& wtab, std::map<int, int>& htab,
+                   std::vector<ResizeImage>& im);
+  bool plan_fused(const std::vector<int32_t>& t, const std::map<int, int>& wtab, const std::map<int, int>& htab);
 };
 int launch_resize(const uint8_t* base, const ResizePlan& rp, uint8_t* out, cudaStream_t stream);
 
