@@ -110,33 +110,42 @@ __global__ void __launch_bounds__(256) batch_composite_kernel(const BatchMosaic*
                                                               int total_cells, const uint8_t* __restrict__ thumbs,
                                                               int tw, int th, const float4* __restrict__ adj) {
   __shared__ float s_bc[2][256];
+  __shared__ float s_unit[256];
   __shared__ uint32_t s_perm[8];
   sector_perm_table(s_perm);
+  tile_unit_table(s_unit);
+  const TileLane lane = tile_lane(tw);
   const int per = (total_cells + gridDim.x - 1) / gridDim.x;
   const int c0 = blockIdx.x * per, c1 = min(total_cells, c0 + per);
   int mi = c0 < c1 ? find_mosaic(mos, nm, c0) : 0;
   int it = 0;
+  // the next cell's material (when of the same mosaic) and adjustment, read a tile ahead
+  float4 next_a = c0 < c1 ? adj[c0] : make_float4(0.0f, 1.0f, 0.0f, 1.0f);
+  int next_g = -1, next_of = -1;  // the cell that next_g is of
   for (int c = c0; c < c1; ++c, ++it) {
     while (mi + 1 < nm && mos[mi + 1].cell_base <= c) ++mi;
     const BatchMosaic& M = mos[mi];
     const int local = c - M.cell_base;
     const bool real = local < M.n;  // else a padding cell
-    const int g = real ? M.final_grid[local] : -1;
+    const int g = !real ? -1 : next_of == c ? next_g : M.final_grid[local];
     const bool adjust = M.strength > 0.0f;
     float* bc = s_bc[it & 1];
-    Adjust a{0.0f, 1.0f, 0.0f, 1.0f};
-    if (adjust && g >= 0) {
-      const float4 a4 = adj[c];
-      a = Adjust{a4.x, a4.y, a4.z, a4.w};
-      tile_bc_table(bc, a);
+    const Adjust a{next_a.x, next_a.y, next_a.z, next_a.w};
+    if (c + 1 < c1) {
+      next_a = adj[c + 1];
+      if (local + 1 < M.n) {
+        next_g = M.final_grid[local + 1];
+        next_of = c + 1;
+      }
     }
+    if (adjust && g >= 0) tile_bc_table(bc, s_unit, a);
     __syncthreads();
     if (!real) continue;
     const size_t pitch = (size_t)M.gw * tw * 3;
     const int cy = local / M.gw, cx = local - cy * M.gw;
     uint8_t* dst = M.out + (size_t)cy * th * pitch + (size_t)cx * tw * 3;
     const uint8_t* src = g >= 0 ? thumbs + (size_t)g * tw * th * 3 : nullptr;
-    composite_tile(src, dst, tw, th, pitch, adjust, a, bc, s_perm);
+    composite_tile(src, dst, tw, th, pitch, lane, adjust, a, bc, s_perm);
   }
 }
 

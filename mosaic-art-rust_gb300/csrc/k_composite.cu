@@ -42,32 +42,45 @@ __global__ void __launch_bounds__(256) composite_kernel(const int32_t* __restric
                                                         const uint8_t* __restrict__ thumbs, int tw, int th,
                                                         const float4* __restrict__ adj, uint8_t* __restrict__ out) {
   __shared__ float s_bc[2][256];
+  __shared__ float s_unit[256];
   __shared__ uint32_t s_perm[8];
   sector_perm_table(s_perm);
+  if (kAdjust) tile_unit_table(s_unit);
   const int n = gw * gh;
   const size_t pitch = (size_t)gw * tw * 3;
-  int it = 0;
+  const TileLane lane = tile_lane(tw);
+  int it = 0, cy = (int)blockIdx.x / gw, cx = (int)blockIdx.x - cy * gw;
+  const int dcy = (int)gridDim.x / gw, dcx = (int)gridDim.x - dcy * gw;
+  // the next tile's material and adjustment, read a tile ahead
+  int next_m = (int)blockIdx.x < n ? grid[blockIdx.x] : -1;
+  float4 next_a = make_float4(0.0f, 1.0f, 0.0f, 1.0f);
+  if (kAdjust && (int)blockIdx.x < n) next_a = adj[blockIdx.x];
   for (int c = blockIdx.x; c < n; c += gridDim.x, ++it) {
-    const int m = grid[c];
-    float* bc = s_bc[it & 1];
-    Adjust a{0.0f, 1.0f, 0.0f, 1.0f};
-    if (kAdjust && m >= 0) {
-      const float4 a4 = adj[c];
-      a = Adjust{a4.x, a4.y, a4.z, a4.w};
-      tile_bc_table(bc, a);
+    const int m = next_m;
+    const Adjust a{next_a.x, next_a.y, next_a.z, next_a.w};
+    if (c + (int)gridDim.x < n) {
+      next_m = grid[c + gridDim.x];
+      if (kAdjust) next_a = adj[c + gridDim.x];
     }
+    float* bc = s_bc[it & 1];
+    if (kAdjust && m >= 0) tile_bc_table(bc, s_unit, a);
     __syncthreads();
-    const int cy = c / gw, cx = c - cy * gw;
     uint8_t* dst = out + (size_t)cy * th * pitch + (size_t)cx * tw * 3;
     const uint8_t* src = m >= 0 ? thumbs + (size_t)m * tw * th * 3 : nullptr;
-    composite_tile(src, dst, tw, th, pitch, kAdjust, a, bc, s_perm);
+    composite_tile(src, dst, tw, th, pitch, lane, kAdjust, a, bc, s_perm);
+    cy += dcy;
+    cx += dcx;
+    if (cx >= gw) {
+      cx -= gw;
+      ++cy;
+    }
   }
 }
 
 // apply_to_image: adjust_pixel on every pixel; for adjustments in
 // adjustment_new's ranges (and a brightness and contrast that are not NaN,
 // so the brightness/contrast table holds channels in [0, 1]) through the
-// composite's arithmetic, the table and adjust_word.
+// composite's arithmetic, the table and adjust_words.
 __global__ void __launch_bounds__(256) adjust_image_kernel(float4 a4, const uint8_t* __restrict__ in, int w, int h,
                                                            int64_t stride, uint8_t* __restrict__ out) {
   __shared__ float s_unit[256];
@@ -84,7 +97,7 @@ __global__ void __launch_bounds__(256) adjust_image_kernel(float4 a4, const uint
     const uint8_t* s = in + (int64_t)y * stride + 3 * x;
     uint8_t* d = out + t * 3;
     if (word) {
-      const uint32_t p = adjust_word(a, s_unit[s[0]], s_unit[s[1]], s_unit[s[2]], s_perm);
+      const uint32_t p = tile_pixel<kTileWord>(s[0], s[1], s[2], a, s_unit, s_perm);
       d[0] = (uint8_t)p;
       d[1] = (uint8_t)(p >> 8);
       d[2] = (uint8_t)(p >> 16);
