@@ -45,6 +45,13 @@ __device__ __forceinline__ int grid_coord(float v, float lo, float inv, int g) {
   return (int)fminf(fmaxf(t, 0.0f), (float)(g - 1));  // NaN -> 0
 }
 
+// A warp's keys: the list form's three buffers, or the other form's flat one
+// (kGatherCap keys, from w.list on).
+struct GridLists {
+  WarpLists w;
+  unsigned long long more[kListCap];
+};
+
 struct Box {
   int x0, x1, y0, y1, z0, z1;  // inclusive bucket ranges
 };
@@ -199,13 +206,20 @@ __device__ __forceinline__ void scan_box(const int* start, int g, const Box& o, 
 
 // ---- the select-then-sort query ------------------------------------------------------------
 // Most queries take this form: their candidate keys are gathered into the
-// warp's flat buffer (the WarpLists memory, kGatherCap keys), the k-th
-// distance among them is found by bisection on the distance bits (a warp
-// count per step), the buffer is cut to the keys at or below it, and one
-// bitonic sort of what is left gives the k smallest keys -- instead of the
-// top-k list's repeated sorts and merges.  A query whose candidates do not fit
-// takes the list form (scan_box + warp_merge), which gives the same keys.
-constexpr int kGatherCap = 3 * kListCap;  // list, tmp and buf of WarpLists, contiguous
+// warp's flat buffer (GridLists, kGatherCap keys), a distance that at least k of
+// them lie within is found by bisection on the distance bits (a warp count per
+// step), the buffer is cut to the keys at or below it, and one bitonic sort of
+// what is left gives the k smallest keys -- instead of the top-k list's repeated
+// sorts and merges.  A query whose candidates do not fit takes the list form
+// (scan_box + warp_merge), which gives the same keys.
+// What bounds it: instructions issued (76% of the slots), of a query's ~4000 about
+// a third the gathering, a third the two bisections, a quarter the sort.
+// Measured, GB300, k = 100, before (exact k-th distances, the sort in shared
+// memory, 384 keys, buckets of 2 entries) -> now: 24 000 queries against 5000
+// entries 0.186 -> 0.110 ms, 470 000 against 10 000 1.88 -> 1.18; 24 000 against
+// 2600, 20 000 and 60 000 entries 0.143, 0.241 and 0.313 (with the new sort
+// alone) -> 0.101, 0.174 and 0.289.  640 keys: 10 000 entries 1.22.
+constexpr int kGatherCap = 4 * kListCap;
 
 // Appends the keys of box o (minus box in, when has_in) whose distance bits
 // are at most dthr to buf[n..); returns the new count (beyond cap: nothing
@@ -271,10 +285,13 @@ __device__ __forceinline__ int gather_box(const int* start, int g, const Box& o,
   return n;
 }
 
-// The smallest distance D (as bits) with at least k of buf[0..n) at or below
-// it (k <= n <= kGatherCap): bisection between the smallest and the largest.
-__device__ uint32_t kth_dist_bits(const unsigned long long* buf, int n, int k, int lane) {
-  constexpr int kPer = kGatherCap / 32;
+// A distance D (as bits) with at least k of buf[0..n) at or below it (k <= n <=
+// 32 kPer), by bisection between the smallest and the largest: the first one met
+// with at most `most` at or below it, else (ties) the smallest there is.  The
+// search's k-th distance only bounds a box, and the sort takes a power of two, so
+// neither needs the k-th exactly (exactly: 26 steps, ~30 instructions each).
+template <int kPer>
+__device__ __forceinline__ uint32_t dist_bound(const unsigned long long* buf, int n, int k, int most, int lane) {
   uint32_t d[kPer];
   uint32_t mn = 0xFFFFFFFFu, mx = 0u;
 #pragma unroll
@@ -292,10 +309,22 @@ __device__ uint32_t kth_dist_bits(const unsigned long long* buf, int n, int k, i
     unsigned c = 0;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) c += d[j] <= mid ? 1u : 0u;
-    if ((int)__reduce_add_sync(kFull, c) >= k) hi = mid;
-    else lo = mid + 1u;
+    const int count = (int)__reduce_add_sync(kFull, c);
+    if (count < k) {
+      lo = mid + 1u;
+    } else {
+      hi = mid;
+      if (count <= most) break;
+    }
   }
-  return lo;
+  return hi;
+}
+__device__ __forceinline__ uint32_t kth_dist_bound(const unsigned long long* buf, int n, int k, int most, int lane) {
+  constexpr int kPer = kGatherCap / 32;
+  static_assert(kPer > 8, "the steps below");
+  if (n <= 128) return dist_bound<4>(buf, n, k, most, lane);
+  if (n <= 256) return dist_bound<8>(buf, n, k, most, lane);
+  return dist_bound<kPer>(buf, n, k, most, lane);
 }
 
 // Keeps the keys of buf[0..n) whose distance bits are at most dthr (in order);
@@ -331,14 +360,14 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
     const float4* __restrict__ queries, int nq, int k, int out_stride, uint32_t* __restrict__ out_idx,
     float* __restrict__ out_dist) {
   extern __shared__ __align__(16) uint8_t smem[];
-  WarpLists* lists = reinterpret_cast<WarpLists*>(smem);
-  int* start = reinterpret_cast<int*>(smem + kGridWarps * sizeof(WarpLists));
+  GridLists* lists = reinterpret_cast<GridLists*>(smem);
+  int* start = reinterpret_cast<int*>(smem + kGridWarps * sizeof(GridLists));
   const LabGrid H = *hdr;
   const int g = H.g, nb = g * g * g;
   for (int i = threadIdx.x; i <= nb; i += blockDim.x) start[i] = start_g[i];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WarpLists& W = lists[warp];
+  WarpLists& W = lists[warp].w;
   const int target = min(H.p, kBoxFactor * k);
   for (int qi = blockIdx.x * kGridWarps + warp; qi < nq; qi += gridDim.x * kGridWarps) {
     const float4 q = queries[qi];
@@ -367,7 +396,7 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
       bool fits = m <= kGatherCap;
       if (fits && m > 0 && !box_is_all(c, g)) {
         // the cube holds >= min(P, k) entries: its k-th distance bounds the search
-        const uint32_t dk = kth_dist_bits(fb, m, min(k, m), lane);
+        const uint32_t dk = kth_dist_bound(fb, m, min(k, m), k + k / 32, lane);
         m = cut_keys(fb, m, dk, lane);
         if (m >= k) {
           const float r = __fsqrt_rn(__uint_as_float(dk));
@@ -385,9 +414,10 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
       }
       if (fits && m > 0) {
         const int kk = min(k, m);
-        const uint32_t d2 = kth_dist_bits(fb, m, kk, lane);
-        m = cut_keys(fb, m, d2, lane);  // the k smallest keys and their ties at the k-th distance
         int mp = 1;
+        while (mp < kk) mp <<= 1;
+        const uint32_t d2 = kth_dist_bound(fb, m, kk, mp, lane);
+        m = cut_keys(fb, m, d2, lane);  // the k smallest keys and some more, at most mp but for ties
         while (mp < m) mp <<= 1;
         if (mp <= kGatherCap) {
           for (int i = m + lane; i < mp; i += 32) fb[i] = kMaxKey;
@@ -430,14 +460,17 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
   }
 }
 
-size_t grid_query_smem(int g) { return kGridWarps * sizeof(WarpLists) + sizeof(int) * ((size_t)g * g * g + 1); }
+size_t grid_query_smem(int g) { return kGridWarps * sizeof(GridLists) + sizeof(int) * ((size_t)g * g * g + 1); }
 
 }  // namespace
 
 int lab_grid_dim(int method, int p, int k) {
   if (p <= 0 || method == kNearestScan) return 0;
   if (method == kNearestAuto && (p < 2048 || p < 16 * k)) return 0;
-  const int g = (int)std::lround(std::cbrt(p / 2.0));
+  // 2.5 entries a bucket: at 2 the first cube holds too few and the box is walked
+  // in more pieces (10 000 entries 1.44 ms, 1.18 at 2.5 and 1.19 at 3), at 3.5 more
+  // first cubes do not fit in the buffer (1.25)
+  const int g = (int)std::lround(std::cbrt(p / 2.5));
   return std::max(1, std::min(kMaxGridDim, g));
 }
 
