@@ -180,7 +180,7 @@ KERNEL_OF_STAGE = {"palette_lab": "region_stats_kernel", "similarity": "similari
 # Stages that are chains of dependent decisions (their bytes are a lower bound;
 # the limit is the latency of one decision), and the data-parallel ones.
 SEQUENTIAL = {"greedy": "latency of one placement decision (row-major walk, sequential by definition)",
-              "anneal": "latency of one round of 16 proposals per chain (32 chains, sequential within a chain)"}
+              "anneal": "latency of one level of a window of 64 proposals (32 chains, sequential within a chain)"}
 DATA_PARALLEL = ["palette_lab", "nearest", "similarity", "composite"]
 
 
