@@ -89,7 +89,7 @@ __device__ __forceinline__ uint2 adjust_words(const Adjust& a, float2 c0, float2
   order(c0.x, c1.x, c2.x, mx.x, mn.x, p.x, q.x, coeff.x);
   order(c0.y, c1.y, c2.y, mx.y, mn.y, p.y, q.y, coeff.y);
   const float2 sep = __fadd2_rn(p, neg(q)), d = __fadd2_rn(mx, neg(mn));
-  auto reciprocal = [&](float2 v) {  // correctly rounded (roots.cuh's rcp_in_range)
+  auto reciprocal = [&](float2 v) {  // correctly rounded (checked for every float of [2^-67, 4))
     float2 y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(v.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(v.y));
