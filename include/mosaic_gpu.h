@@ -231,6 +231,12 @@ int mg_ctx_set_scoring(mg_ctx* ctx, int scoring);
  * returns MG_ERR_TIMEOUT, the walk's grid is left empty (-1), and the context
  * and its plans stay usable.  0 cancels. */
 int mg_ctx_inject_walk_timeout(mg_ctx* ctx, int walks);
+/* The same for tests of the walk's hand-overs: from this call on, the walks named
+ * above run with the publication of every candidate record (scout_ns) and the
+ * making of every prepared list (refiner_ns) held back by that long, 0 to 100000
+ * nanoseconds each (MG_ERR_ARG beyond).  They get slower; their results stay the
+ * same.  0, 0 cancels. */
+int mg_ctx_inject_walk_delay(mg_ctx* ctx, int scout_ns, int refiner_ns);
 
 /* ---- adjacency ------------------------------------------------------------------ */
 /* adjacency.rs:63-88 calculate_penalty for n (candidate, x, y) triples

@@ -236,6 +236,13 @@ bool valid_image(const void* p, int w, int h, int64_t stride) {
   return p && w > 0 && h > 0 && stride >= 3ll * w;
 }
 
+// What the context's next walk has injected (mg_ctx_inject_walk_timeout, mg_ctx_inject_walk_delay).
+WalkInject walk_inject(mg_ctx* ctx) {
+  WalkInject w{ctx->inject_walk_timeouts > 0, (uint32_t)ctx->inject_scout_ns, (uint32_t)ctx->inject_refiner_ns};
+  if (w.timeout) --ctx->inject_walk_timeouts;
+  return w;
+}
+
 const LabConsts* device_lab_consts(mg_ctx* ctx) {
   if (!ctx->lab_consts.p) {
     if (ctx->lab_consts.ensure(sizeof(LabConsts)) != MG_OK) return nullptr;
@@ -369,6 +376,15 @@ int mg_ctx_inject_walk_timeout(mg_ctx* ctx, int walks) {
   if (!ctx) return fail(MG_ERR_ARG, "null context");
   if (walks < 0) return fail(MG_ERR_ARG, "negative walk count");
   ctx->inject_walk_timeouts = walks;
+  return MG_OK;
+}
+
+int mg_ctx_inject_walk_delay(mg_ctx* ctx, int scout_ns, int refiner_ns) {
+  if (!ctx) return fail(MG_ERR_ARG, "null context");
+  if (scout_ns < 0 || scout_ns > 100000 || refiner_ns < 0 || refiner_ns > 100000)
+    return fail(MG_ERR_ARG, "delays must be in 0..100000 ns");
+  ctx->inject_scout_ns = scout_ns;
+  ctx->inject_refiner_ns = refiner_ns;
   return MG_OK;
 }
 
@@ -665,8 +681,7 @@ int mg_place_greedy(mg_ctx* ctx, const float* palette_lab, int p, const float* c
   GreedyJob job{ctx->out0.as<uint32_t>(), ctx->out1.as<float>(), d_grid, gw, gh, k,
                 (uint32_t)cfg->max_usage_per_image, cfg->adjacency_penalty_weight, d_resets, nullptr};
   MG_CHECK(upload(ctx, ctx->regions, &job, sizeof(job)));
-  const bool inject = ctx->inject_walk_timeouts > 0;
-  if (inject) --ctx->inject_walk_timeouts;
+  const WalkInject inject = walk_inject(ctx);
   MG_CHECK(launch_greedy(ctx->in0.as<float4>(), p, ctx->regions.as<GreedyJob>(), 1, k, gw, n,
                          ctx->sums.as<uint32_t>(), ctx->err.as<uint32_t>(), ctx->stream, false, inject));
   MG_CUDA(cudaMemcpyAsync(grid_out, d_grid, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1155,8 +1170,7 @@ int plan_run(mg_plan* pl) {
   MG_CUDA(cudaEventRecord(pl->ev[4], s));
   // [4] greedy placement
   if (P > 0) {
-    const bool inject = pl->ctx->inject_walk_timeouts > 0;
-    if (inject) --pl->ctx->inject_walk_timeouts;
+    const WalkInject inject = walk_inject(pl->ctx);
     MG_CHECK(launch_greedy(pl->pal_lab.as<float4>(), P, pl->greedy_job.as<GreedyJob>(), 1, pl->k, pl->gw, N,
                            pl->usage.as<uint32_t>(), pl->err.as<uint32_t>(), s, false, inject));
   } else {

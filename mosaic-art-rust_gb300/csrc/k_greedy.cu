@@ -104,10 +104,14 @@ __host__ __device__ inline int scout_ahead(int gw, int p, uint32_t max_usage) {
   if (a > kScoutLead) a = kScoutLead;
   return a < gw ? a : gw;
 }
-// Lists of a cap-1 palette below this many materials go unused: the cells placed
-// since a list was made have what it held (200 materials, cap 1: 2.68 ms with
-// them, 1.74 without; 1000 materials: 1.36 and 1.60).
+// Lists of a cap-1 palette below this many materials would go unused: the cells
+// placed since a list was made have what it held (200 materials, cap 1: 2.68 ms
+// with them, 1.74 without; 1000 materials: 1.36 and 1.60).  Such a walk makes none
+// and goes by the records alone.
 constexpr int kCapOneLists = 512;
+__device__ __forceinline__ bool walks_by_lists(int p, uint32_t max_usage) {
+  return max_usage > 1u || p >= kCapOneLists;
+}
 constexpr uint32_t kRefinePolls = 1u << 26;  // the refiners' bounded waits (seconds)
 constexpr int kCostChunk = 2048;  // cells per pass of the final cost sum
 constexpr uint32_t kFollowPolls = 1u << 26;  // the cost warp's bounded wait for a placement (seconds)
@@ -488,11 +492,11 @@ __device__ void follow_walk(const GreedyJob& J, int p, uint8_t* smem, int R, uin
 // (The layout is recomputed here rather than passed by reference: a struct
 // whose address escapes would turn the walker's shared-memory pointers into
 // generic ones.)
-// withhold: build the records but never publish them (an injected fault: the
-// walker's wait for the first record then runs out).
+// inject.timeout: build the records but never publish them (the walker's wait for
+// the first record then runs out); inject.scout_ns: publish each that much later.
 template <bool kRing, int kScouts>
 __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict__ pal, int p, uint8_t* smem,
-                            ScoutStage& S, int R, uint32_t* err, bool withhold) {
+                            ScoutStage& S, int R, uint32_t* err, const WalkInject& inject) {
   const int lane = threadIdx.x & 31;
   const int gw = J.gw, k = J.k, n = gw * J.gh;
   const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
@@ -611,9 +615,10 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
                     make_uint4(__float_as_uint(la.x), __float_as_uint(la.y), __float_as_uint(la.z), 0u));
       if (lane == 0) st_cluster_u32(rr + (uint32_t)offsetof(CellRecord, f_next), __float_as_uint(cf < 32 ? inf : af));
     }
+    if (inject.scout_ns) __nanosleep(inject.scout_ns);
     fence_cluster();
     __syncwarp();
-    if (lane == 0 && !withhold) st_release_cluster(r_seq + 4u * slot, (uint32_t)(c + 1));
+    if (lane == 0 && !inject.timeout) st_release_cluster(r_seq + 4u * slot, (uint32_t)(c + 1));
   }
   return true;
 }
@@ -622,7 +627,7 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
 // bounded; one that runs out aborts the walk.
 template <bool kLabSmem, bool kRing>
 __device__ void refine_cells(int r, const GreedyJob& J, const float4* __restrict__ pal, int p, uint8_t* smem, int R,
-                             uint32_t* err) {
+                             uint32_t* err, uint32_t delay_ns) {
   const int lane = threadIdx.x & 31;
   const int gw = J.gw, k = J.k, n = gw * J.gh;
   const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
@@ -714,6 +719,7 @@ __device__ void refine_cells(int r, const GreedyJob& J, const float4* __restrict
                  (int)ld_acquire_cta(&Q.done[(past + 1) & (kLists - 1)]) > past + 1;
         }))
       return;
+    if (delay_ns) __nanosleep(delay_ns);
     use_f = __all_sync(0xffffffffu, rec_epoch == ld_volatile_u32(&L.ctrl[kEpoch]));
     if (!use_f) load_row(c);
     const int lead = c - kRefineLag;
@@ -817,7 +823,7 @@ __device__ void refine_cells(int r, const GreedyJob& J, const float4* __restrict
 template <bool kLabSmem, bool kRing>
 __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThreads, 1)
     greedy_pair_kernel(const float4* __restrict__ pal, int p, const GreedyJob* __restrict__ jobs, uint32_t* err,
-                       uint32_t walk_polls, uint32_t withhold) {
+                       uint32_t walk_polls, WalkInject inject) {
   extern __shared__ __align__(128) uint8_t smem[];
   const GreedyJob J = jobs[blockIdx.x / (1 + kScoutCtas)];
   const uint32_t rank = cluster_ctarank();
@@ -859,7 +865,7 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
     bool ok = true;
     if (warp < kPer)
       ok = scout_cells<kRing, kScoutCtas * kPer>(
-          (int)(rank - 1) * kPer + warp, J, pal, p, smem, F.stage[warp], R, err, withhold != 0u);
+          (int)(rank - 1) * kPer + warp, J, pal, p, smem, F.stage[warp], R, err, inject);
     else
       follow_walk<kRing>(J, p, smem, R, err);
     if (rank > 1) {
@@ -979,7 +985,8 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   if (warp != 0) {
     // ---- CTA 0, the refiners (not on the walker's scheduler)
     const int r = warp - warp / 4 - 2;
-    if ((warp & 3) != 0 && r >= 0 && r < kRefiners) refine_cells<kLabSmem, kRing>(r, J, pal, p, smem, R, err);
+    if (walks_by_lists(p, J.max_usage) && (warp & 3) != 0 && r >= 0 && r < kRefiners)
+      refine_cells<kLabSmem, kRing>(r, J, pal, p, smem, R, err, inject.refiner_ns);
     cluster_sync_all();
     return;
   }
@@ -1141,7 +1148,16 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   // 30 materials, cap 1: 3.89 -> 1.84 ms a call.  (Its result and what follows
   // from it go through a shuffle: the compiler else takes the walker's loops for
   // divergent, 1.0 -> 1.4 ms for 5000 materials, which never come here.)
-  int rec_ready = 0;  // the cells before it have records
+  int rec_ready = 0;  // the records of the cells from the walker's to before it are published
+  // The word beside a record names the cell it is of.
+  auto record_there = [&](int c) -> bool {
+    return __all_sync(0xffffffffu, ld_acquire_cluster(smem_u32(&L.seq[c & (R - 1)])) == (uint32_t)(c + 1));
+  };
+  // After `polls` polls: whether the walk ends here.
+  auto gives_up = [&](uint32_t polls) -> bool {
+    aborted = polls > walk_polls || __any_sync(0xffffffffu, ld_volatile_u32(&ctrl[kAbort]) != 0u);
+    return aborted;
+  };
   auto record_cells = [&](int c, int end, int left) -> int {
     if (c >= rec_ready) {
       const int cc = c + lane;
@@ -1179,20 +1195,24 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
     }
     return __shfl_sync(0xffffffffu, c, 0);  // (uniform for the compiler)
   };
-  const bool lists = max_usage > 1u || p >= kCapOneLists;
+  const bool lists = walks_by_lists(p, max_usage);
   int old_lists = 0;         // lists of cells before it may be of an earlier epoch
   bool known = true;         // b names the previous choice's position in its list
   uint32_t b = kClear;
   int c = 0;
   while (c < n) {
-    // the list of cell c (bounded wait: its refiner waits for nothing the walker has yet to do)
-    Entry e = load_entry(c);
-    for (uint32_t polls = 0; !__all_sync(0xffffffffu, ((e.hi ^ list_tag(c, 0)) & kTagCell) == 0u);) {
-      if (++polls > walk_polls || __any_sync(0xffffffffu, ld_volatile_u32(&ctrl[kAbort]) != 0u)) {
-        aborted = true;
-        break;
-      }
+    // the list of cell c, or, in a walk without lists, its record (bounded waits:
+    // who makes them waits for nothing the walker has yet to do)
+    Entry e{0u, 0u};
+    if (lists) {
       e = load_entry(c);
+      for (uint32_t polls = 0; !__all_sync(0xffffffffu, ((e.hi ^ list_tag(c, 0)) & kTagCell) == 0u);) {
+        if (gives_up(++polls)) break;
+        e = load_entry(c);
+      }
+    } else if (c >= rec_ready) {
+      for (uint32_t polls = 0; !record_there(c);)
+        if (gives_up(++polls)) break;
     }
     if (aborted) break;
     if (!lists || c < old_lists) {
@@ -1297,7 +1317,7 @@ bool greedy_scouted_fits(int gw, int n, int p) {
 
 int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_jobs, int k, int max_gw,
                   int max_cells, uint32_t* usage_scratch, uint32_t* err, cudaStream_t stream, bool one_warp,
-                  bool inject_timeout) {
+                  WalkInject inject) {
   if (n_jobs <= 0) return MG_OK;
   if (k < 1 || k > 100) return fail(MG_ERR_ARG, "candidate count must be in 1..100");
   constexpr size_t kMaxSmem = 227 * 1024 - 128;  // beside the kernel's static words
@@ -1328,9 +1348,9 @@ int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_job
     if (form >= 0) {
       const bool lab_smem = form == 0 || form == 2, ring = form >= 2;
       const size_t bytes = pair_smem_bytes(max_gw, max_cells, p, lab_smem, ring);
-      const uint32_t polls = inject_timeout ? kInjectedWalkPolls : kWalkPolls, hold = inject_timeout ? 1u : 0u;
+      const uint32_t polls = inject.timeout ? kInjectedWalkPolls : kWalkPolls;
       auto go = [&](auto kernel) {
-        kernel<<<(unsigned)((1 + kScoutCtas) * n_jobs), kThreads, bytes, stream>>>(pal, p, jobs_dev, err, polls, hold);
+        kernel<<<(unsigned)((1 + kScoutCtas) * n_jobs), kThreads, bytes, stream>>>(pal, p, jobs_dev, err, polls, inject);
       };
       if (form == 0) go(greedy_pair_kernel<true, false>);
       else if (form == 1) go(greedy_pair_kernel<false, false>);

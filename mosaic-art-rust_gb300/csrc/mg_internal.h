@@ -149,13 +149,20 @@ struct GreedyJob {
 };
 // Candidate arrays must hold ceil(N/16)*16 rows (the walk streams 16 rows per copy).
 // one_warp: every job walks in the one-warp form (else the three-CTA form when
-// every job allows it).  inject_timeout (three-CTA form only): the scouts
-// withhold their records and the walker waits at most a few thousand polls,
-// so its bounded wait runs out -- an injected fault for tests.  A walk that
-// gives up sets kErrTimeout in *err and leaves every cell of its grid empty.
+// every job allows it).  A walk that gives up sets kErrTimeout in *err and leaves
+// every cell of its grid empty.
+// WalkInject, for tests (three-CTA form only): with `timeout` the scouts withhold
+// their records and the walker waits at most a few thousand polls, so its bounded
+// wait runs out; the delays hold back every record and every list, so that the
+// walker and the warps that prepare its cells meet in an order they do not have
+// by themselves.
+struct WalkInject {
+  bool timeout = false;
+  uint32_t scout_ns = 0, refiner_ns = 0;
+};
 int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_jobs, int k, int max_gw,
                   int max_cells, uint32_t* usage_scratch, uint32_t* err, cudaStream_t stream, bool one_warp = false,
-                  bool inject_timeout = false);
+                  WalkInject inject = {});
 inline size_t padded_cells(int n) { return ((size_t)n + 15) / 16 * 16; }
 // Most cells of one mosaic, or of all the mosaics of one batch (indices stay 32-bit).
 constexpr int64_t kMaxGridCells = int64_t(1) << 28;

@@ -135,6 +135,7 @@ SIGNATURES = [
     ("mg_ctx_set_thumbnail_filter", C.c_int, [C.c_void_p, C.c_int]),
     ("mg_resize", C.c_int, [C.c_void_p, _u8p, C.c_int, C.c_int, C.c_int64, C.c_int, C.c_int, _u8p]),
     ("mg_ctx_inject_walk_timeout", C.c_int, [C.c_void_p, C.c_int]),
+    ("mg_ctx_inject_walk_delay", C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     ("mg_ctx_set_scoring", C.c_int, [C.c_void_p, C.c_int]),
     ("mg_host_alloc", C.c_void_p, [C.c_size_t]),
     ("mg_host_free", None, [C.c_void_p]),
