@@ -212,9 +212,10 @@ constexpr int kLists = 16;      // ring of lists (more than kRefineLag + 3)
 constexpr uint32_t kRankOpen = 14, kClear = 1u << 24;
 constexpr uint32_t kNotThere = 0xFFFFu;  // the packed word of an entry whose list is not there
 constexpr int kResetLog = 128;  // more resets than cells between the walker and its followers
-// The tag bits of a list: a slot holds cell c's list or still the one a turn of
-// the ring before; between a list's making and its use lie fewer than 32 cells,
-// so fewer than 32 resets.
+// The tag bits of a list tell cell c's from the one a turn of the ring before (cell
+// c - kLists), not from older ones: a reader of cell c's slot knows that the list of
+// c - kLists has been there (the walker's `behind`).  Between a list's making and
+// its use lie fewer than 32 cells, so fewer than 32 resets.
 constexpr uint32_t kTagMask = 0xF0820000u, kTagCell = 0x00800000u;
 __device__ __forceinline__ uint32_t list_tag(int c, uint32_t epoch) {
   return (epoch << 28) | ((epoch & 16u) << 13) | (((uint32_t)c & kLists) ? kTagCell : 0u);
@@ -1021,11 +1022,13 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   struct Cur {
     uint32_t key, ti, ui;
     bool f;  // the key is the record's f entry (its epoch is the walk's)
+    bool there;  // the record was published when it was read
   };
   auto record_entry = [&](int c) {
-    (void)ld_acquire_cta(&Q.seq[c & (kLists - 1)]);  // its refiner saw the record published
-    const CellRecord& Rc = rec[c & (R - 1)];
     Cur r;
+    // (the refiner that sets this word saw the record published)
+    r.there = ld_acquire_cta(&Q.seq[c & (kLists - 1)]) == (uint32_t)(c + 1);
+    const CellRecord& Rc = rec[c & (R - 1)];
     r.f = Rc.epoch == epoch;
     r.key = r.f ? Rc.kf[lane] : Rc.kr[lane];
     r.ti = r.key & 0xFFFFu;
@@ -1197,6 +1200,8 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   };
   const bool lists = walks_by_lists(p, max_usage);
   int old_lists = 0;         // lists of cells before it may be of an earlier epoch
+  constexpr int kTurn = kLists - 2, kNoneBehind = 0x7FFF0000;  // (fast_cells reads the list two cells on)
+  int behind = kNoneBehind;  // the first cell passed by a run whose list the walker has not seen
   bool known = true;         // b names the previous choice's position in its list
   uint32_t b = kClear;
   int c = 0;
@@ -1205,6 +1210,17 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
     // who makes them waits for nothing the walker has yet to do)
     Entry e{0u, 0u};
     if (lists) {
+      // A cell passed by its list has been in its slot; a run from records leaves cells
+      // behind whose lists may be late.  Until those are done, the walk stays
+      // within a turn of the ring of the first of them.
+      if (c + 4 > behind + kTurn) {
+        const int j = c - kLists + (lane & (kLists - 1));
+        for (uint32_t polls = 0;
+             !__all_sync(0xffffffffu, j < behind || (int)ld_acquire_cta(&Q.done[j & (kLists - 1)]) > j);)
+          if (gives_up(++polls)) break;
+        if (aborted) break;
+        behind = __shfl_sync(0xffffffffu, kNoneBehind, 0);
+      }
       e = load_entry(c);
       for (uint32_t polls = 0; !__all_sync(0xffffffffu, ((e.hi ^ list_tag(c, 0)) & kTagCell) == 0u);) {
         if (gives_up(++polls)) break;
@@ -1217,15 +1233,19 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
     if (aborted) break;
     if (!lists || c < old_lists) {
       const int c0 = c;
-      c = record_cells(c, min(c + gw - x, lists ? old_lists : n), x == 0 ? -1 : last);
+      c = record_cells(c, min(c + gw - x, lists ? min(old_lists, behind + kTurn) : n), x == 0 ? -1 : last);
       __syncwarp();
       if (c > c0) {
+        behind = __shfl_sync(0xffffffffu, min(behind, c0 + 1), 0);
         x += c - c0;
         if (x == gw) x = 0;
         last = __shfl_sync(0xffffffffu, kRing ? (int)(ring[(c - 1) & cmask] & 0xFFFFu) : (int)grid16[c - 1], 0);
+        // its place in the list of cell c - 1, if that is there: its maker sets seq
+        // when the slot has held the list of the turn before
+        const bool made = __all_sync(0xffffffffu, ld_acquire_cta(&Q.seq[(c - 1) & (kLists - 1)]) == (uint32_t)c);
         const Entry before = load_entry(c - 1);
         const unsigned at = __ballot_sync(0xffffffffu, lane < kList && (before.hi & 0xFFFFu) == (uint32_t)last);
-        known = at != 0u && __all_sync(0xffffffffu, ((before.hi ^ list_tag(c - 1, 0)) & kTagCell) == 0u);
+        known = made && at != 0u && __all_sync(0xffffffffu, ((before.hi ^ list_tag(c - 1, 0)) & kTagCell) == 0u);
         b = kClear | (known ? (uint32_t)(__ffs(at) - 1) << 25 : 0u) | (uint32_t)last;
         continue;
       }
@@ -1234,8 +1254,9 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
     if (lists && fresh && (x == 0 || known)) {
       const int c0 = c;
       if (x == 0) b |= 0xFFFFu;  // no left neighbour
-      if (max_usage < 127u) c = fast_cells(std::false_type{}, c, c + gw - x, b, e);
-      else c = fast_cells(std::true_type{}, c, c + gw - x, b, e);
+      const int end = min(c + gw - x, behind + kTurn);
+      if (max_usage < 127u) c = fast_cells(std::false_type{}, c, end, b, e);
+      else c = fast_cells(std::true_type{}, c, end, b, e);
       __syncwarp();
       if (c > c0) {
         last = (int)(b & 0xFFFFu);
@@ -1247,7 +1268,12 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
     }
     // ---- cell c from its record, or in full
     const bool row_start = x == 0;
-    const Cur cu = record_entry(c);
+    Cur cu = record_entry(c);
+    for (uint32_t polls = 0; !__all_sync(0xffffffffu, cu.there || !lists);) {
+      if (gives_up(++polls)) break;
+      cu = record_entry(c);
+    }
+    if (aborted) break;
     const uint32_t key = __reduce_min_sync(
         0xffffffffu, cu.ui < max_usage && (row_start || (int)cu.ti != last) ? cu.key : 0xFFFFFFFFu);
     int t = (int)(key & 0xFFFFu);

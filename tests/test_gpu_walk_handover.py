@@ -35,6 +35,16 @@ def test_records_alone(ctx, orc, gw, p, scout_ns):
                scout_ns, 0)
 
 
+@pytest.mark.parametrize("refiner_ns", [0, 500, 2000, 20000])
+@pytest.mark.parametrize("p,cap", [(5, 2), (16, 2), (40, 2), (120, 2), (9, 3), (300, 2), (700, 1)])
+@pytest.mark.parametrize("gw", [40, 100])
+def test_late_lists(ctx, orc, gw, p, cap, refiner_ns):
+    """Lists that come late, with resets within their lead of one another and beyond it."""
+    for seed in range(4):
+        _check(ctx, orc, seed * 1013 + p, p, gw, 20, cap, [0.25, 1.0, 0.0, 3.0][seed], [0.3, 1.0, 0.3, 0.05][seed],
+               0 if seed < 2 else 900, refiner_ns)
+
+
 def test_delay_arguments(ctx):
     from mosaic_gpu import _capi
 
