@@ -150,14 +150,19 @@ struct ScoutStage {
   float df[32], dr[32];
 };
 
-// Records live in a ring.  A scout writes cell c's record once the walker has
-// placed cell c - lead (lead = min(gw, kScoutLead)), so the walker is past
-// every record up to c - lead and reads at most two ahead of its cell; a ring
-// of more than lead + 3 slots keeps the slot of record c - R free.
-__host__ __device__ inline int ring_size(int gw) {
+// Records live in a ring of R slots.  A scout writes cell c's record once the
+// walker has placed cell c - ahead, and that is when the slot's last one, of cell
+// c - R, must have no reader any more.  The walker is past it and reads two ahead
+// of its cell at most.  A refiner may be later than the walker, which goes kTurn
+// cells past one whose list it has not seen, at most: R >= ahead + kTurn.  Where a
+// ring of that size does not fit, ahead is shorter (rows of 28 cells, a ring of 32
+// for 64: 0.45 -> 0.60 ms a call of 2800 cells, 30 materials, cap 2).
+constexpr int kLists = 16;         // ring of the prepared lists (below)
+constexpr int kTurn = kLists - 2;  // (fast_cells reads the list two cells on)
+__host__ __device__ inline int ring_size(int gw, bool roomy) {
   const int lead = gw < kScoutLead ? gw : kScoutLead;
   int r = 32;
-  while (r < lead + 4) r <<= 1;
+  while (r < lead + (roomy ? kTurn : 4)) r <<= 1;
   return r;
 }
 
@@ -208,7 +213,6 @@ constexpr int kList = 8;
 constexpr int kRefiners = 17;   // warps 2, 3, 5, 6, 7, 9, ... of the walker's CTA
 constexpr int kRefineLag = 12;
 constexpr int kEarly = 3;       // entries that must be clear for the first form (2 to 8 differ by 3%)
-constexpr int kLists = 16;      // ring of lists (more than kRefineLag + 3)
 constexpr uint32_t kRankOpen = 14, kClear = 1u << 24;
 constexpr uint32_t kNotThere = 0xFFFFu;  // the packed word of an entry whose list is not there
 constexpr int kResetLog = 128;  // more resets than cells between the walker and its followers
@@ -239,8 +243,8 @@ static_assert(sizeof(ListShared) % 16 == 0, "16-byte aligned parts");
 __host__ __device__ inline size_t cells_bytes(int gw, int n, bool ring) {
   return ring ? (size_t)cell_ring_size(gw) * 4 : align16((size_t)n * 2);
 }
-__host__ __device__ inline size_t walker_smem_bytes(int gw, int n, int p, bool lab_smem, bool ring) {
-  const int R = ring_size(gw);
+__host__ __device__ inline size_t walker_smem_bytes(int gw, int n, int p, bool lab_smem, bool ring, bool roomy) {
+  const int R = ring_size(gw, roomy);
   size_t b = 16 + sizeof(ListShared) + (size_t)R * sizeof(CellRecord) + (size_t)R * 4;
   b += cells_bytes(gw, n, ring);
   b += align16(((size_t)p + 1) * 4);
@@ -270,8 +274,8 @@ __host__ __device__ inline size_t scout_cta_smem_bytes(int gw, int p) {
   return (size_t)kScoutWarpsMax * sizeof(ScoutStage) + (size_t)kCostChunk * 8 + 16 + align16((size_t)p * 4) +
          (size_t)cell_ring_size(gw) * 2;
 }
-__host__ __device__ inline size_t pair_smem_bytes(int gw, int n, int p, bool lab_smem, bool ring) {
-  const size_t a = walker_smem_bytes(gw, n, p, lab_smem, ring), b = scout_cta_smem_bytes(gw, p);
+__host__ __device__ inline size_t pair_smem_bytes(int gw, int n, int p, bool lab_smem, bool ring, bool roomy = false) {
+  const size_t a = walker_smem_bytes(gw, n, p, lab_smem, ring, roomy), b = scout_cta_smem_bytes(gw, p);
   return a > b ? a : b;
 }
 
@@ -505,7 +509,7 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
   const uint32_t max_usage = J.max_usage;
   const bool use_pen = J.weight > 0.0f;
   const float two_w = __fmul_rn(2.0f, J.weight);
-  const int ahead = scout_ahead(gw, p, max_usage);
+  const int ahead = min(scout_ahead(gw, p, max_usage), R - kTurn);
   const int nr = (k + 31) >> 5;
   const float inf = __int_as_float(0x7f800000);
   const unsigned lt = (1u << lane) - 1u;
@@ -534,7 +538,7 @@ __device__ bool scout_cells(int s, const GreedyJob& J, const float4* __restrict_
     // placements cap dozens of the nearest materials; a record built a whole
     // row ahead would list none left).  The walker read that cell's record
     // before placing it (the placement depends on it), so the walker is done
-    // with the ring slot this record reuses (the ring holds more than gw records).
+    // with the ring slot this record reuses, and so are the refiners (ring_size).
     const int lead = c - ahead;
     for (uint32_t polls = 0;
          lead >= 0 && !__all_sync(0xffffffffu, (int)ld_acquire_cta(&F.ctl[kFollowed]) > lead);) {
@@ -824,7 +828,7 @@ __device__ void refine_cells(int r, const GreedyJob& J, const float4* __restrict
 template <bool kLabSmem, bool kRing>
 __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThreads, 1)
     greedy_pair_kernel(const float4* __restrict__ pal, int p, const GreedyJob* __restrict__ jobs, uint32_t* err,
-                       uint32_t walk_polls, WalkInject inject) {
+                       uint32_t walk_polls, bool roomy, WalkInject inject) {
   extern __shared__ __align__(128) uint8_t smem[];
   const GreedyJob J = jobs[blockIdx.x / (1 + kScoutCtas)];
   const uint32_t rank = cluster_ctarank();
@@ -833,7 +837,7 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   // a convergence step: 138 against 86 cycles a cell in a copy of the loop)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int gw = J.gw, gh = J.gh, k = J.k, n = gw * gh;
-  const int R = ring_size(gw);
+  const int R = ring_size(gw, roomy);
   const WalkerLayout L = walker_layout(smem, gw, n, p, R, kRing);
   if (rank == 0) {
     for (int i = threadIdx.x; i <= p; i += blockDim.x) {
@@ -1200,7 +1204,7 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   };
   const bool lists = walks_by_lists(p, max_usage);
   int old_lists = 0;         // lists of cells before it may be of an earlier epoch
-  constexpr int kTurn = kLists - 2, kNoneBehind = 0x7FFF0000;  // (fast_cells reads the list two cells on)
+  constexpr int kNoneBehind = 0x7FFF0000;
   int behind = kNoneBehind;  // the first cell passed by a run whose list the walker has not seen
   bool known = true;         // b names the previous choice's position in its list
   uint32_t b = kClear;
@@ -1373,10 +1377,11 @@ int launch_greedy(const float4* pal, int p, const GreedyJob* jobs_dev, int n_job
     const int form = fit[0] ? 0 : fit[1] ? 1 : fit[2] ? 2 : fit[3] ? 3 : -1;
     if (form >= 0) {
       const bool lab_smem = form == 0 || form == 2, ring = form >= 2;
-      const size_t bytes = pair_smem_bytes(max_gw, max_cells, p, lab_smem, ring);
+      const bool roomy = pair_smem_bytes(max_gw, max_cells, p, lab_smem, ring, true) <= kMaxSmem;
+      const size_t bytes = pair_smem_bytes(max_gw, max_cells, p, lab_smem, ring, roomy);
       const uint32_t polls = inject.timeout ? kInjectedWalkPolls : kWalkPolls;
       auto go = [&](auto kernel) {
-        kernel<<<(unsigned)((1 + kScoutCtas) * n_jobs), kThreads, bytes, stream>>>(pal, p, jobs_dev, err, polls, inject);
+        kernel<<<(unsigned)((1 + kScoutCtas) * n_jobs), kThreads, bytes, stream>>>(pal, p, jobs_dev, err, polls, roomy, inject);
       };
       if (form == 0) go(greedy_pair_kernel<true, false>);
       else if (form == 1) go(greedy_pair_kernel<false, false>);

@@ -45,6 +45,25 @@ def test_late_lists(ctx, orc, gw, p, cap, refiner_ns):
                0 if seed < 2 else 900, refiner_ns)
 
 
+@pytest.mark.parametrize("refiner_ns", [0, 300, 1000, 4000, 20000])
+@pytest.mark.parametrize("p,cap", [(5, 2), (12, 2), (20, 3), (160, 2)])
+@pytest.mark.parametrize("gw", WIDTHS)
+def test_records_written_again(ctx, orc, gw, p, cap, refiner_ns):
+    """Runs from records beside refiners that are late for theirs: at rows of 28 and 60 cells a
+    slot of the ring is another cell's once the walker is four cells past it."""
+    for seed in range(4):
+        _check(ctx, orc, seed * 1019 + p, p, gw, 26, cap, [0.25, 1.0, 0.0, 3.0][seed], [0.3, 1.0, 0.3, 0.05][seed],
+               0, refiner_ns)
+
+
+@pytest.mark.parametrize("refiner_ns", [0, 4000])
+@pytest.mark.parametrize("gw", [28, 60])
+def test_tight_ring(ctx, orc, gw, refiner_ns):
+    """A palette beside which only the smaller ring of records fits: they are made less far ahead."""
+    for drift in (0.0, 0.05):
+        _check(ctx, orc, gw, 40000 if gw == 28 else 30000, gw, 16, 1, 0.25, drift, 0, refiner_ns)
+
+
 def test_delay_arguments(ctx):
     from mosaic_gpu import _capi
 
