@@ -147,6 +147,7 @@ __device__ __forceinline__ uint32_t tile_pixel(uint32_t b0, uint32_t b1, uint32_
 
 // A thread's place in a tile of `per_row` items a row: its first item and the
 // step to its next one; the same for every tile, so the divisions are made once.
+// (A tile may hold more than 2^31 bytes: its bytes are walked by pointer.)
 struct TileLane {
   int per_row, row, col, drow, dcol;
 };
@@ -184,9 +185,10 @@ __device__ __forceinline__ void tile_pixels(const uint8_t* __restrict__ src, uin
     }
   };
   if ((tw & 3) == 0) {
-    for (; row < th; step()) {
+    // a tile's groups are contiguous: a thread's next one is blockDim.x of them on
+    for (const uint8_t* group = src + 12 * threadIdx.x; row < th; step(), group += 12 * blockDim.x) {
       uint32_t* d = reinterpret_cast<uint32_t*>(dst + row * pitch + 12 * col);
-      const uint32_t* s = reinterpret_cast<const uint32_t*>(src + 12 * (row * lane.per_row + col));
+      const uint32_t* s = reinterpret_cast<const uint32_t*>(group);
       const uint32_t w0 = __ldg(s), w1 = __ldg(s + 1), w2 = __ldg(s + 2);
       if (kMode == kTileCopy) {
         d[0] = w0;
@@ -217,10 +219,12 @@ __device__ __forceinline__ void tile_pixels(const uint8_t* __restrict__ src, uin
     }
     return;
   }
-  for (; row < th; step()) {  // pairs; a row of odd width ends in a pixel of its own
+  // pairs; a row of odd width ends in a pixel of its own, three bytes short of a pair
+  const int lost = 3 * (tw & 1);
+  const uint8_t* s = src + 6 * threadIdx.x - lost * row;
+  for (int from = row; row < th; from = row, step(), s += 6 * (int)blockDim.x - lost * (row - from)) {
     const int x = 2 * col;
     uint8_t* d = dst + row * pitch + 3 * x;
-    const uint8_t* s = src + 3 * (row * tw + x);
     const bool two = x + 1 < tw;
     const uint32_t l0 = s[0], l1 = s[1], l2 = s[2];
     const uint2 p = tile_pixels2<kMode>(l0, l1, l2, two ? s[3] : l0, two ? s[4] : l1, two ? s[5] : l2, a, s_bc, s_perm);
