@@ -351,7 +351,9 @@ typedef struct mg_result {
 void mg_request_default(mg_request* req);
 /* One complete job from host buffers to host buffers.  Inputs in pinned host
  * memory (mg_host_alloc), or in any host memory where the GPU reads through the
- * host's page tables, are read in place over the CPU-GPU link.  A grid holds
+ * host's page tables, are read in place over the CPU-GPU link: they must stay as
+ * they are (mapped, and their files as long as they are) until the call returns.
+ * Memory that cannot be read when the call begins is MG_ERR_ARG.  A grid holds
  * at most 2^28 cells and an output row at most 2^31 / 3 pixels (MG_ERR_ARG
  * beyond; a batch's cells together obey the same cell limit). */
 int mg_generate(mg_ctx* ctx, const mg_request* req, mg_result* res);

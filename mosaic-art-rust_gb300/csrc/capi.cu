@@ -156,8 +156,8 @@ const void* device_view(const void* p) {
 // walks the host's page tables itself, so nothing is registered, copied or moved
 // first.  Worth it for mg_generate, which reads each input once or twice: a copy
 // from pageable memory takes the host ~10 us a material and its bytes at the
-// staging rate (33 materials 678 -> 208 us a call, 112 materials 2.56 -> 0.56 ms,
-// 500 materials 5.4 -> 0.70 ms).
+// staging rate (33 materials 678 -> 211 us a call, 112 materials 2.56 -> 0.56 ms,
+// 500 materials 5.4 -> 0.71 ms).
 bool reads_pageable(int device) {
   int access = 0, tables = 0;
   if (cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, device) != cudaSuccess ||
@@ -168,9 +168,11 @@ bool reads_pageable(int device) {
   return access != 0 && tables != 0;
 }
 
-// device_view; with `pageable` also the address itself of host memory that CUDA
-// does not know (`known`: whether it does).
-const void* input_view(const void* p, bool pageable, bool* known = nullptr) {
+// device_view of `rows` rows of `bytes` bytes, `stride` apart; with a probe also the
+// address itself of host memory that CUDA does not know (`known`: whether it does).
+// The rows are added to the probe then: no kernel may be given them before its end()
+// has said that they can be read.
+const void* input_view(const void* p, size_t bytes, size_t rows, size_t stride, ReadProbe* probe, bool* known = nullptr) {
   cudaPointerAttributes a;
   if (known) *known = false;
   if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -179,7 +181,9 @@ const void* input_view(const void* p, bool pageable, bool* known = nullptr) {
   }
   if (known) *known = a.type == cudaMemoryTypeHost;
   if (a.type == cudaMemoryTypeHost) return a.devicePointer;
-  return pageable && a.type == cudaMemoryTypeUnregistered ? p : nullptr;
+  if (!probe || a.type != cudaMemoryTypeUnregistered) return nullptr;
+  probe->add(p, bytes, rows, stride);
+  return p;
 }
 
 // Device views of caller buffers for one setup: the first query of a pinned
@@ -187,18 +191,19 @@ const void* input_view(const void* p, bool pageable, bool* known = nullptr) {
 // other buffers inside it -- hundreds of materials packed in one pinned block,
 // say -- need no query.  Kept for one call only: allocations change between calls.
 struct ViewCache {
-  bool pageable = false;
+  ReadProbe* probe = nullptr;
   struct Range {
     uintptr_t lo, hi;
     intptr_t delta;  // device address - host address
   };
   std::vector<Range> ranges;
-  const void* view(const void* p, size_t bytes) {
+  const void* view(const void* p, size_t row_bytes, size_t rows, size_t stride) {
     const uintptr_t u = (uintptr_t)p;
+    const size_t bytes = stride * (rows - 1) + row_bytes;
     for (const Range& r : ranges)
       if (u >= r.lo && u + bytes <= r.hi) return (const void*)(u + r.delta);
     bool known;
-    const void* d = input_view(p, pageable, &known);
+    const void* d = input_view(p, row_bytes, rows, stride, probe, &known);
     if (!known) return d;
     using GetAttr = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
     static GetAttr get = [] {
@@ -967,8 +972,8 @@ int plan_setup(mg_plan* pl, mg_ctx* ctx, const mg_request* r, bool zero_copy) {
   // target
   const size_t trow = 3ull * pl->W;
   const int64_t tstride = r->target_stride ? r->target_stride : (int64_t)trow;
-  const bool pageable = pl->zero_copy && reads_pageable(ctx->device);
-  const void* tdev = pl->zero_copy ? input_view(r->target, pageable) : nullptr;
+  ReadProbe* probe = pl->zero_copy && reads_pageable(ctx->device) && ctx->probe.begin() ? &ctx->probe : nullptr;
+  const void* tdev = pl->zero_copy ? input_view(r->target, trow, pl->H, tstride, probe) : nullptr;
   if (tdev) {
     pl->target_ptr = static_cast<const uint8_t*>(tdev);
     pl->target_stride = tstride;
@@ -1003,15 +1008,14 @@ int plan_setup(mg_plan* pl, mg_ctx* ctx, const mg_request* r, bool zero_copy) {
   pl->h_regions.resize(std::max(P, 1));
   std::vector<const void*> mdev(std::max(P, 1), nullptr);
   ViewCache views;
-  views.pageable = pageable;
+  views.probe = probe;
   int64_t off = 0;
   for (int i = 0; i < P; ++i) {
     const int m = pl->selected[i];
     const int64_t st = r->material_stride ? r->material_stride[m] : 3ll * r->material_w[m];
     if (!valid_image(r->materials[m], r->material_w[m], r->material_h[m], st))
       return fail(MG_ERR_ARG, "invalid material " + std::to_string(m));
-    mdev[i] = pl->zero_copy ? views.view(r->materials[m], (size_t)st * (r->material_h[m] - 1) + 3ull * r->material_w[m])
-                            : nullptr;
+    mdev[i] = pl->zero_copy ? views.view(r->materials[m], 3ull * r->material_w[m], r->material_h[m], st) : nullptr;
     if (mdev[i]) {
       pl->h_regions[i] = Region{(int64_t)(uintptr_t)mdev[i], r->material_w[m], r->material_h[m], st};
     } else {
@@ -1038,8 +1042,17 @@ int plan_setup(mg_plan* pl, mg_ctx* ctx, const mg_request* r, bool zero_copy) {
   pl->thumb_filter = ctx->thumb_filter;
   if (pl->device_thumbs && pl->thumb_filter == MG_THUMB_LANCZOS3)
     MG_CHECK(pl->resize.build(pl->h_regions.data(), P, pl->tw, pl->th, s));
+  const void* thdev = nullptr;
+  if (!pl->device_thumbs && pl->zero_copy && P > 0) {
+    bool known;
+    thdev = input_view(r->thumbnails, 0, 0, 0, probe, &known);
+    if (thdev && !known)
+      for (int i = 0; i < P; ++i) probe->add(r->thumbnails + tb * pl->selected[i], tb, 1, tb);
+  }
+  if (probe && !probe->end())
+    return probe->error() == EFAULT ? fail(MG_ERR_ARG, "an input image lies in memory that cannot be read")
+                                    : fail(MG_ERR_STATE, "cannot tell whether the input images can be read");
   if (!pl->device_thumbs) {
-    const void* thdev = pl->zero_copy && P > 0 ? input_view(r->thumbnails, pageable) : nullptr;
     if (thdev) {
       // One gather kernel pulls the selected thumbnails across the link.
       std::vector<int64_t> src(P);

@@ -3,6 +3,7 @@
 #pragma once
 #include <vector>
 
+#include "host_readable.h"
 #include "mg_internal.h"
 
 namespace mg {
@@ -15,6 +16,7 @@ struct mg_ctx {
   cudaStream_t side = nullptr;  // forked from `stream` for stages that can overlap, joined back
   mg::DevBuf in0, in1, in2, out0, out1, out2, sums, regions, err, lab_consts;
   mg_plan* gen_plan = nullptr;
+  mg::ReadProbe probe;                    // mg_generate: whether inputs that it reads in place can be read
   int nearest_method = mg::kNearestAuto;  // MG_NEAREST_*
   int scoring = 0;                        // MG_SCORING_*
   int inject_walk_timeouts = 0;           // mg_ctx_inject_walk_timeout: walks left to fail on purpose
