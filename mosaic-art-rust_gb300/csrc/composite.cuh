@@ -14,6 +14,7 @@
 // words.
 #pragma once
 #include "mg_internal.h"
+#include "roots.cuh"
 
 namespace mg {
 
@@ -89,14 +90,9 @@ __device__ __forceinline__ uint2 adjust_words(const Adjust& a, float2 c0, float2
   order(c0.x, c1.x, c2.x, mx.x, mn.x, p.x, q.x, coeff.x);
   order(c0.y, c1.y, c2.y, mx.y, mn.y, p.y, q.y, coeff.y);
   const float2 sep = __fadd2_rn(p, neg(q)), d = __fadd2_rn(mx, neg(mn));
-  auto reciprocal = [&](float2 v) {  // correctly rounded (checked for every float of [2^-67, 4))
-    float2 y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(v.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(v.y));
-    return __ffma2_rn(y, __ffma2_rn(neg(v), y, pair(1.0f)), y);
-  };
-  const float2 yd = reciprocal(make_float2(fmaxf(d.x, 1e-20f), fmaxf(d.y, 1e-20f)));
-  const float2 ym = reciprocal(make_float2(fmaxf(mx.x, 1e-20f), fmaxf(mx.y, 1e-20f)));
+  // (the divisors are at most 1)
+  const float2 yd = rcp2_in_range(make_float2(fmaxf(d.x, 1e-20f), fmaxf(d.y, 1e-20f)));
+  const float2 ym = rcp2_in_range(make_float2(fmaxf(mx.x, 1e-20f), fmaxf(mx.y, 1e-20f)));
   float2 hd = __fmul2_rn(sep, yd), s = __fmul2_rn(d, ym);
   hd = __ffma2_rn(__ffma2_rn(neg(hd), d, sep), yd, hd);
   s = __ffma2_rn(__ffma2_rn(neg(s), mx, d), ym, s);

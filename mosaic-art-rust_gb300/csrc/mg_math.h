@@ -517,7 +517,9 @@ MG_HD bool adjust_word_applies(const Adjust& a) {
          a.saturation >= 0.0f && a.saturation <= 2.0f;
 }
 
-// adjust_unit for adjustments with adjust_word_applies, the output bytes as
+// adjust_unit for adjustments with adjust_word_applies, one pixel of what the
+// composite's adjust_words (composite.cuh) does for two -- there the quotients by
+// reciprocals --, as host code for the proof over all byte triples; the output bytes as
 // one word (r | g << 8 | b << 16; byte 3 is not part of the result).  `perm`
 // holds sector_perm(i) at index i (0..7; device code: shared memory).
 // Rearranged further without changing a result:

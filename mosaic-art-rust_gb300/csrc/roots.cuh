@@ -1,12 +1,12 @@
-// roots.cuh -- correctly rounded square root and reciprocal for the adjacency
-// weights and the similarity matrix, without the range branches of the general
-// forms: inside [1e-30, 1e30] nothing can overflow, underflow or lose bits, so
-// the hardware's approximate reciprocal square root (or reciprocal) and one
+// roots.cuh -- the adjacency weights' square root and reciprocal and the
+// composite's reciprocal, correctly rounded, without the range branches of the
+// general forms: in the ranges given nothing can overflow, underflow or lose bits,
+// so the hardware's approximate reciprocal square root (or reciprocal) and one
 // correction by fused multiply-adds of the exact residual gives the rounded
 // result (the last step of Markstein's method, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 1990).
-// Equal to __fsqrt_rn for all 1 671 934 059 floats of [1e-30, 1e30] and to
-// __frcp_rn for all of [1, 1e30] (every float compared on the GB300).
+// tests/test_gpu_roots.py compares every float of those ranges on the device: with
+// __frcp_rn, and the weights with __frcp_rn(__fsqrt_rn(s) + 1).
 // Two chains of these interleave, where the general forms' branches run one
 // after the other.
 #pragma once
@@ -14,18 +14,18 @@
 
 namespace mg {
 
-// s in [1e-30, 1e30].
-__device__ __forceinline__ float sqrt_in_range(float s) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
-  const float g = __fmul_rn(s, y);
-  return __fmaf_rn(__fmaf_rn(-g, g, s), __fmul_rn(0.5f, y), g);
-}
 // x in [1, 1e30].
 __device__ __forceinline__ float rcp_in_range(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
+// Two at once in packed arithmetic, each in [2^-67, 4).
+__device__ __forceinline__ float2 rcp2_in_range(float2 v) {
+  float2 y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(v.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(v.y));
+  return __ffma2_rn(y, __ffma2_rn(make_float2(-v.x, -v.y), y, make_float2(1.0f, 1.0f)), y);
 }
 
 // 1 / (distance + 1) of adjacency.rs:83 from a squared distance, any float: the
