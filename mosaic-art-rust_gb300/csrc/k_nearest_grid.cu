@@ -39,6 +39,7 @@ constexpr int kGridThreads = kGridWarps * 32;
 constexpr int kBoxFactor = 1;   // the first cube holds >= kBoxFactor * k entries
 constexpr int kMaxGridDim = 24; // start[] of 24^3 + 1 ints stays in shared memory
 constexpr unsigned kFull = 0xffffffffu;
+constexpr uint32_t kInfBits = 0x7f800000u;  // distances from here on bound no box
 
 __device__ __forceinline__ int grid_coord(float v, float lo, float inv, int g) {
   const float t = floorf(__fmul_rn(__fsub_rn(v, lo), inv));
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
         // the cube holds >= min(P, k) entries: its k-th distance bounds the search
         const uint32_t dk = kth_dist_bound(fb, m, min(k, m), k + k / 32, lane);
         m = cut_keys(fb, m, dk, lane);
-        if (m >= k) {
+        if (m >= k && dk < kInfBits) {
           const float r = __fsqrt_rn(__uint_as_float(dk));
           const float R = __fadd_rn(__fmul_rn(r, 1.001f), 1e-3f);
           const Box o{grid_coord(__fsub_rn(q.x, R), H.lo[0], H.inv[0], g), grid_coord(__fadd_rn(q.x, R), H.lo[0], H.inv[0], g),
@@ -406,7 +407,8 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
                       grid_coord(__fsub_rn(q.z, R), H.lo[2], H.inv[2], g), grid_coord(__fadd_rn(q.z, R), H.lo[2], H.inv[2], g)};
           m = gather_box(start, g, o, c, true, sorted, q, fb, m, kGatherCap, dk, lane);
         } else {
-          // fewer than k in the cube (palette below k): every entry counts
+          // fewer than k in the cube (palette below k), or fewer that are not NaN (those
+          // lie in bucket 0, and sort behind every number): every entry counts
           const Box all{0, g - 1, 0, g - 1, 0, g - 1};
           m = gather_box(start, g, all, c, true, sorted, q, fb, m, kGatherCap, 0xFFFFFFFFu, lane);
         }
@@ -443,7 +445,7 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
         // the cube holds >= min(P, k) entries: len == k unless P < k
         const float r = __fsqrt_rn(__uint_as_float((uint32_t)(thr >> 32)));
         const float R = __fadd_rn(__fmul_rn(r, 1.001f), 1e-3f);
-        const Box o = len < k ? Box{0, g - 1, 0, g - 1, 0, g - 1} : Box{grid_coord(__fsub_rn(q.x, R), H.lo[0], H.inv[0], g), grid_coord(__fadd_rn(q.x, R), H.lo[0], H.inv[0], g),
+        const Box o = len < k || (uint32_t)(thr >> 32) >= kInfBits ? Box{0, g - 1, 0, g - 1, 0, g - 1} : Box{grid_coord(__fsub_rn(q.x, R), H.lo[0], H.inv[0], g), grid_coord(__fadd_rn(q.x, R), H.lo[0], H.inv[0], g),
                     grid_coord(__fsub_rn(q.y, R), H.lo[1], H.inv[1], g), grid_coord(__fadd_rn(q.y, R), H.lo[1], H.inv[1], g),
                     grid_coord(__fsub_rn(q.z, R), H.lo[2], H.inv[2], g), grid_coord(__fadd_rn(q.z, R), H.lo[2], H.inv[2], g)};
         scan_box(start, g, o, c, true, sorted, q, W, len, nbuf, thr, k, lane);
