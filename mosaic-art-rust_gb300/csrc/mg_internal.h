@@ -6,6 +6,7 @@
 #include <atomic>
 #include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/mosaic_gpu.h"
@@ -94,8 +95,9 @@ struct ResizePlan {
   void release();
 
  private:
-  int build_images(const Region* regions, std::vector<int32_t>& t, std::map<int, int>& wtab, std::map<int, int>& htab,
-                   std::vector<ResizeImage>& im);
+  using ResizeWeights = std::map<std::pair<int, int>, std::vector<int32_t>>;
+  int build_images(const Region* regions, ResizeWeights& weights, std::vector<int32_t>& t, std::map<int, int>& wtab,
+                   std::map<int, int>& htab, std::vector<ResizeImage>& im);
   bool plan_fused(const std::vector<int32_t>& t, const std::map<int, int>& wtab, const std::map<int, int>& htab);
 };
 int launch_resize(const uint8_t* base, const ResizePlan& rp, uint8_t* out, cudaStream_t stream);
