@@ -367,7 +367,7 @@ int mg_resize(mg_ctx* ctx, const uint8_t* rgb, int w, int h, int64_t stride, int
   MG_CHECK(ctx->out2.ensure(bytes));
   const Region r{0, w, h, stride};
   if (ctx->thumb_filter == MG_THUMB_LANCZOS3) {
-    MG_CHECK(ctx->resize.build(&r, 1, dw, dh, ctx->stream));
+    MG_CHECK(ctx->resize.build(&r, 1, dw, dh, device_view(rgb) != nullptr, ctx->stream));
     MG_CHECK(launch_resize(src, ctx->resize, ctx->out2.as<uint8_t>(), ctx->stream));
   } else {
     MG_CHECK(upload(ctx, ctx->regions, &r, sizeof(r)));
@@ -1040,8 +1040,10 @@ int plan_setup(mg_plan* pl, mg_ctx* ctx, const mg_request* r, bool zero_copy) {
   MG_CHECK(pl->thumbs.ensure(tb * std::max(P, 1)));
   pl->device_thumbs = r->thumbnails == nullptr;
   pl->thumb_filter = ctx->thumb_filter;
-  if (pl->device_thumbs && pl->thumb_filter == MG_THUMB_LANCZOS3)
-    MG_CHECK(pl->resize.build(pl->h_regions.data(), P, pl->tw, pl->th, s));
+  if (pl->device_thumbs && pl->thumb_filter == MG_THUMB_LANCZOS3) {
+    const bool over_link = 2 * std::count_if(mdev.begin(), mdev.end(), [](const void* v) { return v != nullptr; }) > P;
+    MG_CHECK(pl->resize.build(pl->h_regions.data(), P, pl->tw, pl->th, over_link, s));
+  }
   const void* thdev = nullptr;
   if (!pl->device_thumbs && pl->zero_copy && P > 0) {
     bool known;

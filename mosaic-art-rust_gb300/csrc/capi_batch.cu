@@ -114,7 +114,7 @@ int palette_setup(mg_palette* pl, mg_ctx* ctx, const mg_palette_desc* d) {
       MG_CUDA(cudaMemcpyAsync(pl->thumbs.as<uint8_t>() + tb * i, d->thumbnails + tb * pl->selected[i], tb,
                               cudaMemcpyHostToDevice, s));
   } else if (P > 0 && ctx->thumb_filter == MG_THUMB_LANCZOS3) {
-    MG_CHECK(pl->resize.build(pl->h_regions.data(), P, pl->tw, pl->th, s));
+    MG_CHECK(pl->resize.build(pl->h_regions.data(), P, pl->tw, pl->th, false, s));
     MG_CHECK(launch_resize(pl->mats.as<uint8_t>(), pl->resize, pl->thumbs.as<uint8_t>(), s));
   } else if (P > 0) {
     MG_CHECK(launch_thumbnails(pl->mats.as<uint8_t>(), pl->regions.as<Region>(), P, pl->tw, pl->th,

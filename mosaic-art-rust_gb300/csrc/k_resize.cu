@@ -20,9 +20,9 @@
 // the CPU oracle computes the same bytes.  Parity with fast_image_resize's own
 // fixed-point choices is not pinned (the crate is not here to run).
 //
-// Two forms:
-//  - resize_fused_kernel: both passes in one CTA per image (per band of output
-//    rows where images are few), the source and the 8-bit intermediate in shared
+// Two forms (choose_bands):
+//  - resize_fused_kernel: both passes in one CTA per image or band of output rows,
+//    the source and the 8-bit intermediate in shared
 //    memory.  What bounds it is the multiply-adds: two passes of ~6 * scale taps
 //    a sample, and at a byte a tap an extraction for each.  So bytes are kept
 //    four to a word along the dimension the next pass sums over -- the source by
@@ -31,13 +31,14 @@
 //    of a channel.  The sums are integers, so the split changes nothing.  A
 //    thread makes four rows of a column, which share the weights it reads.
 //  - resize_h_kernel, resize_v_kernel: the passes one after the other, a thread a
-//    sample, the intermediate in global memory; for images whose rows, weights
+//    sample, the intermediate in global memory; also for images whose rows, weights
 //    and intermediate do not fit in shared memory (kMaxFusedWords).
 //
 // Layout of a table for in -> out.  Two-kernel form: [out, kmax], then out (first
 // tap, tap count) pairs, then out rows of kmax weights.  Fused form: [nw], then
 // out (first word << 16 | words) of four taps, then out rows of (3 nw) | 1 words
 // (odd: rows start in different banks), words p0, p1, p2 of each four taps.
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <vector>
@@ -136,10 +137,79 @@ bool append_fused(int in, int out, const std::vector<int32_t>& o, std::vector<in
   return true;
 }
 
+// ---- which form, and how many bands
+// Neither form is the faster one everywhere: the fused one does a band by one CTA,
+// which is slow where there are few images and each is scaled down far (one image of
+// 1000 x 1000 to 16 x 12: 1290 us in two bands, 240 in two kernels), and a band reads
+// 6 * scale source rows beside its own, which counts twice where the sources come over
+// the CPU-GPU link (14 images of 1000 x 1000 to 64 x 48 there: 640 and 330 us); the
+// other one does a tap a byte (400 of 500 x 500 to 16 x 12: 317 and 1430 us) and
+// fetches bytes again and again from the link once its rows overflow the L1 caches.
+// So both are estimated, the fused one for each number of bands.  The constants
+// (microseconds) are fits to measured times of 739 sets of 1 to 2000 images of 40 to
+// 1500 pixels a side, thumbnails of 8 to 200, in all forms; the choice is within 5%
+// of the best form on the average, with the sources on the device and over the link.
+struct ResizeShape {
+  double n, w, h, tw, th;  // images, their mean size, the thumbnail's
+  int sms;
+};
 constexpr int kFusedThreads = 256;
 constexpr int kFusedPerSm = 3;          // CTAs of an SM the shared memory is planned for
 constexpr int kFusedWords = 18 * 1024;  // ... in words; more only where one image needs it
 constexpr int kMaxFusedWords = 50 * 1024;
+
+double taps(double in, double out) { return in == out ? 1.0 : 6.0 * std::max(in / out, 1.0) + 1.0; }
+
+double fused_us(const ResizeShape& s, int bands, bool link) {
+  const double rows = std::ceil(s.th / bands);  // of output, by a CTA
+  const double scale = std::max(s.h / s.th, 1.0), beside = bands == 1 ? 0 : bands == 2 ? 3 : 6;
+  const double in_rows = std::min(s.h, rows * s.h / s.th + beside * scale);
+  const double xw = s.w == s.tw ? 1.0 : std::floor(taps(s.w, s.tw) / 4) + 2, yw = s.h == s.th ? 1.0 : std::floor(taps(s.h, s.th) / 4) + 2;
+  const double quads = std::min(std::ceil(s.h / 4), in_rows / 4 + 1);  // groups of four source rows
+  const double fixed = s.tw * (3 * xw + 1) + rows * (3 * yw + 1) + 3 * s.tw * (quads + 1), group = 12 * (s.w / 4 + 1);
+  const double at_once = std::max(1.0, std::min(quads, std::floor((kFusedWords - fixed) / group)));
+  const double words = fixed + at_once * group;
+  if (words > kMaxFusedWords) return 1e30;
+  const double steps = std::ceil(quads / at_once);
+  const double h_ops = std::ceil(quads / steps * s.tw / kFusedThreads) * steps * xw * 36;
+  const double v_ops = std::ceil(rows * s.tw / kFusedThreads) * yw * 9;
+  const double loads = in_rows * s.w / 4 / kFusedThreads;
+  const double cta = link ? 0.00108 * h_ops + 0.0155 * v_ops + 0.869 * loads + 0.734 * steps
+                          : 0.00106 * h_ops + 0.0162 * v_ops + 0.397 * loads + 0.535 * steps;
+  const double turns = std::ceil(s.n * bands / s.sms);  // CTAs an SM, some of them at a time
+  const int resident = (int)std::max(1.0, std::min({(double)kFusedPerSm, std::floor(227.0 * 1024 / (4 * words + 1024)), turns}));
+  const double rate = resident == 1 ? 1.0 : resident == 2 ? 1.53 : 1.78;
+  const double read = s.n * s.w * 3 * std::min(bands * s.h, s.h + (bands - 1) * 6 * scale);  // bytes
+  return link ? 7.3 + cta * turns / rate + 3.04e-6 * read : 6.0 + cta * turns / rate;
+}
+
+double two_kernels_us(const ResizeShape& s, bool link) {
+  const double tx = taps(s.w, s.tw), ty = taps(s.h, s.th);
+  const double blocks = std::min(16.0, std::ceil(s.h * s.tw / 256));  // an image's
+  auto pass = [](double chain, double all) { return std::pow(std::pow(chain, 4) + std::pow(all, 4), 0.25); };
+  const double h_chain = std::ceil(s.h * s.tw / (256 * blocks)) * tx, h_all = 1e-6 * s.n * s.h * s.tw * tx;
+  const double v_chain = std::ceil(s.th * s.tw / (256 * blocks)) * ty, v_all = 1e-6 * s.n * s.th * s.tw * ty;
+  // KB of source rows that an SM's blocks are in at a time: what its L1 has to hold
+  const double kb = std::min(8.0, s.n * blocks / s.sms) * std::max(1.0, 256 / s.tw) * 3 * s.w / 1024;
+  const double mb = 1e-6 * s.n * s.w * s.h * 3;
+  return link ? 11.3 + pass(0.104 * h_chain, 0.0) + pass(0.127 * v_chain, 1.17 * v_all) + 4.19 * mb * (1 + std::pow(kb / 57.2, 1.79))
+              : 10.2 + pass(0.0904 * h_chain, 0.0347 * h_all) + pass(0.0790 * v_chain, 0.969 * v_all) + 0.812 * mb * std::pow(kb, 0.345);
+}
+
+// The bands of the fastest form by these, 0: two kernels.
+int choose_bands(const ResizeShape& s, bool link) {
+  int best = 0;
+  double best_us = two_kernels_us(s, link);
+  for (int b : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48}) {
+    if (b > std::max(1.0, s.th / 2)) break;
+    const double us = fused_us(s, b, link);
+    if (us < best_us) {
+      best = b;
+      best_us = us;
+    }
+  }
+  return best;
+}
 
 // The band's rows of output.
 __host__ __device__ inline int band_row(int b, int bands, int th) { return (int)((int64_t)b * th / bands); }
@@ -396,16 +466,9 @@ int ResizePlan::build_images(const Region* regions, ResizeWeights& weights, std:
   return MG_OK;
 }
 
-// Bands and shared memory of the fused form; false when they do not fit.  An
-// image is one CTA where two an SM come of that; fewer images are cut into bands
-// of output rows (each needs 6 * scale source rows more than its own, so no band
-// is below six rows of output, 6 * scale of source).
+// Shared memory of the fused form in `bands` bands; false when it does not fit.
 bool ResizePlan::plan_fused(const std::vector<int32_t>& t, const std::map<int, int>& wtab,
                             const std::map<int, int>& htab) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return false;
-  bands = std::max(1, std::min((2 * sms + n - 1) / n, th / 6));
   int64_t hw = 0, vw = 0, rows = 0, pw = 1;
   for (const auto& e : wtab) {
     hw = std::max(hw, (int64_t)tw * ((3 * t[e.second]) | 1));
@@ -428,7 +491,7 @@ bool ResizePlan::plan_fused(const std::vector<int32_t>& t, const std::map<int, i
   return true;
 }
 
-int ResizePlan::build(const Region* regions, int n_images, int tw_, int th_, cudaStream_t s) {
+int ResizePlan::build(const Region* regions, int n_images, int tw_, int th_, bool over_link, cudaStream_t s) {
   if (n_images <= 0) {
     n = 0;
     return MG_OK;
@@ -441,10 +504,19 @@ int ResizePlan::build(const Region* regions, int n_images, int tw_, int th_, cud
   ResizeWeights weights;
   std::map<int, int> wtab, htab;  // source width / height -> table offset
   std::vector<ResizeImage> im((size_t)n);
-  fused = true;
+  int dev = 0;
+  ResizeShape shape{(double)n, 0.0, 0.0, (double)tw, (double)th, 0};
+  MG_CUDA(cudaGetDevice(&dev));
+  MG_CUDA(cudaDeviceGetAttribute(&shape.sms, cudaDevAttrMultiProcessorCount, dev));
+  for (int i = 0; i < n; ++i) {
+    shape.w += (double)regions[i].w / n;
+    shape.h += (double)regions[i].h / n;
+  }
+  bands = choose_bands(shape, over_link);
+  fused = bands > 0;
   MG_CHECK(build_images(regions, weights, t, wtab, htab, im));
   if (fused) fused = plan_fused(t, wtab, htab);
-  if (!fused) {
+  if (!fused && bands > 0) {
     t.clear();
     wtab.clear();
     htab.clear();

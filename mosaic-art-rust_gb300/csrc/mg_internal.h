@@ -91,7 +91,8 @@ struct ResizePlan {
   // both passes in one kernel: the CTAs of an image, and their shared memory in words
   bool fused = false;
   int bands = 1, hw_words = 0, vw_words = 0, src_words = 0, inter_pitch = 0;
-  int build(const Region* regions, int n_images, int tw, int th, cudaStream_t s);
+  // over_link: the images lie in host memory, read over the CPU-GPU link
+  int build(const Region* regions, int n_images, int tw, int th, bool over_link, cudaStream_t s);
   void release();
 
  private:
