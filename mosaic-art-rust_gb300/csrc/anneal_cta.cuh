@@ -446,21 +446,41 @@ __device__ __forceinline__ void anneal_chain_cta(const float4* __restrict__ pal,
     if (J.initial_cost) {
       current = __ldcg(J.initial_cost);
     } else {
+      // 32 cells at a time, their cells read two steps ahead of the sum and their
+      // Lab one (216 x 160 cells, 36 iterations, a whole call: 1104 -> 800 us).
       auto lab = [&](int i) -> float4 { return kLabSmem ? s_lab[i] : __ldg(pal + i); };
-      current = 0.0f;
-      for (int c0 = 0; c0 < n; c0 += 32) {
-        const int c = c0 + lane;
-        float tr = 0.0f, td = 0.0f;
+      struct Cells {
+        int cur, right, down;
+      };
+      auto cells = [&](int c0) -> Cells {
+        const int c = c0 + lane, x = c % gw, y = c / gw;
+        Cells v{-1, -1, -1};
         if (c < n) {
-          const int x = c % gw, y = c / gw;
-          const int cur = __ldcg(J.grid_in + c);
-          if (cur >= 0) {
-            const float4 lc = lab(cur);
-            const int r = x < gw - 1 ? __ldcg(J.grid_in + c + 1) : -1, d = y < gh - 1 ? __ldcg(J.grid_in + c + gw) : -1;
-            if (r >= 0) tr = wgt(lc, lab(r));
-            if (d >= 0) td = wgt(lc, lab(d));
-          }
+          v.cur = __ldcg(J.grid_in + c);
+          if (x < gw - 1) v.right = __ldcg(J.grid_in + c + 1);
+          if (y < gh - 1) v.down = __ldcg(J.grid_in + c + gw);
         }
+        return v;
+      };
+      struct Labs {
+        float4 cur, right, down;
+        bool r, d;
+      };
+      auto labs = [&](const Cells& v) -> Labs {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        Labs l{zero, zero, zero, v.cur >= 0 && v.right >= 0, v.cur >= 0 && v.down >= 0};
+        if (v.cur >= 0) l.cur = lab(v.cur);
+        if (l.r) l.right = lab(v.right);
+        if (l.d) l.down = lab(v.down);
+        return l;
+      };
+      current = 0.0f;
+      Labs now = labs(cells(0));
+      Cells next = cells(32);
+      for (int c0 = 0; c0 < n; c0 += 32) {
+        const float tr = now.r ? wgt(now.cur, now.right) : 0.0f, td = now.d ? wgt(now.cur, now.down) : 0.0f;
+        now = labs(next);
+        next = cells(c0 + 64);
         const int cnt = min(32, n - c0);
         for (int s = 0; s < cnt; ++s) {
           current = __fadd_rn(current, __shfl_sync(0xffffffffu, tr, s));
