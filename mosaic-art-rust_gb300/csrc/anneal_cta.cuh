@@ -86,6 +86,7 @@ struct ChainShared {
   float temps[kProducers][kWindow + 4];    // the window's first temperature after 0, 1, ... coolings
   float temp[kProducers];                  // first temperature of the window in the slot
   float sums[kWindow];                     // the running cost after each proposal of a window
+  int first[4];                            // greedy descent: the lowest level that accepts, in [0] and [1] by turns
 };
 
 // Behind it: the writers table (kProducers x 2 x writer_slots words), the
@@ -378,6 +379,7 @@ __device__ __forceinline__ void evaluate_windows(const float4* __restrict__ pal,
   Desc next{};
   if (windows > 0) next = take(0);
   int o = 0;  // the window's outcome slot
+  int turn = 0;
   for (long long w = 0; w < windows; ++w) {
     const Desc D = next;
     Outcome& O = S.out[o];
@@ -385,22 +387,44 @@ __device__ __forceinline__ void evaluate_windows(const float4* __restrict__ pal,
     {
       const uint16_t g1 = s_grid[D.p1], g2 = s_grid[D.p2], a1 = s_grid[D.n1], a2 = s_grid[D.n2];
       if (w + 1 < windows) next = take(w + 1);
-      // Greedy descent ends in windows that accept nothing, and then what every
-      // level finds on the grid as it is stands: one pass (else the levels above
-      // 0 are done again).  20 000 iterations on 12 x 9 cells 1.86 -> 1.31 ms; with
-      // a temperature, where windows accept, the levels alone are faster (1.53
-      // against 1.70 ms for 100 000 on 179 x 134).
       const bool act = kGreedy ? D.level >= 0 : D.level == 0;
       bool accept = false;
-      if (__any_sync(0xffffffffu, act)) accept = decide(D, g1, g2, a1, a2, O, act, !kGreedy || D.level == 0);
+      if (__any_sync(0xffffffffu, act)) accept = decide(D, g1, g2, a1, a2, O, act, !kGreedy);
       if (D.level < 0 && dir == 0) {
         O.delta[q] = 0.0f;
         O.flags[q] = 0u;
       }
-      if (kGreedy && D.levels > 1 && !bar_any(kBarEval, kEval, accept)) continue;
+      // Greedy descent ends in windows that accept nothing, and then what every
+      // level finds on the grid as it is stands: one pass.  Else that holds up to
+      // the lowest level that accepts; its swaps are made and the levels above it
+      // are looked at again, all at once.  (With a temperature, where windows
+      // accept at most levels, one level after the other is faster: 1.53 against 1.70 ms
+      // for 100 000 on 179 x 134.)  5000 iterations on 8 x 6 cells, 8 chains, a whole
+      // call: 562 -> 240 us (471 in rounds of 16 proposals).
+      if (kGreedy) {
+        for (;;) {
+          const int lowest = __reduce_min_sync(0xffffffffu, accept ? D.level : kWindow);
+          if (lane == 0 && lowest < kWindow) atomicMin(&S.first[turn], lowest);
+          if (!bar_any(kBarEval, kEval, accept)) break;
+          const int done = S.first[turn];
+          if (accept && D.level == done) {
+            const uint16_t t = s_grid[D.p1];  // (no other swap of the level touches these)
+            s_grid[D.p1] = s_grid[D.p2];
+            s_grid[D.p2] = t;
+          }
+          turn ^= 1;
+          if (tid == 0) S.first[turn] = kWindow;
+          bar_sync(kBarEval, kEval);  // the level's swaps are in place
+          if (done + 1 >= D.levels) break;
+          accept = false;
+          if (__any_sync(0xffffffffu, D.level > done))
+            accept = decide(D, s_grid[D.p1], s_grid[D.p2], s_grid[D.n1], s_grid[D.n2], O, D.level > done, false);
+        }
+        continue;
+      }
     }
     for (int l = 1; l < D.levels; ++l) {
-      if (l > 1 || !kGreedy) bar_sync(kBarEval, kEval);
+      bar_sync(kBarEval, kEval);
       if (__any_sync(0xffffffffu, D.level == l))
         decide(D, s_grid[D.p1], s_grid[D.p2], s_grid[D.n1], s_grid[D.n2], O, D.level == l, true);
     }
@@ -428,6 +452,7 @@ __device__ __forceinline__ void anneal_chain_cta(const float4* __restrict__ pal,
     s_grid[i] = g < 0 ? kNone16 : (uint16_t)g;
   }
   for (int i = tid; i < kProducers * 2 * writer_slots; i += kThreads) writers[i] = 0u;
+  if (tid < 2) S.first[tid] = kWindow;
   __syncthreads();
   const long long windows = (J.iters + kWindow - 1) / kWindow;
 
