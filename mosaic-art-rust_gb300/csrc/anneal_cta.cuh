@@ -263,7 +263,10 @@ __device__ __forceinline__ void produce_windows(const AnnealJob& J, int chain, l
       float lo = 0.0f, hi = 0.0f, t = 0.0f;
       if (!greedy_only) {
         t = temps[__popc(live[h] & below) + (h ? __popc(live[0]) : 0)];
-        const bool ok = u[h] > 0.0f && t >= 1e-30f && t <= 1e30f;
+        // T in [+0, 1e30], compared as bits (minus zero accepts everything).  Below
+        // 1e-30 the bounds are not exact to 1e-4 any more, but need not be: a delta that
+        // is not zero is 2^-90 at least (the weights' last bits), far beyond them.
+        const bool ok = u[h] > 0.0f && __float_as_uint(t) <= __float_as_uint(1e30f);
         const float theta = -t * __logf(u[h]), margin = 1e-4f * t;
         lo = ok ? fmaxf(theta - margin, 0.0f) : -inf;
         hi = ok ? theta + margin : inf;
