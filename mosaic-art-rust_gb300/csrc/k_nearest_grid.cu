@@ -34,8 +34,6 @@
 namespace mg {
 namespace {
 
-constexpr int kGridWarps = 16;
-constexpr int kGridThreads = kGridWarps * 32;
 constexpr int kBoxFactor = 1;   // the first cube holds >= kBoxFactor * k entries
 constexpr int kMaxGridDim = 24; // start[] of 24^3 + 1 ints stays in shared memory
 constexpr unsigned kFull = 0xffffffffu;
@@ -46,12 +44,19 @@ __device__ __forceinline__ int grid_coord(float v, float lo, float inv, int g) {
   return (int)fminf(fmaxf(t, 0.0f), (float)(g - 1));  // NaN -> 0
 }
 
-// A warp's keys: the list form's three buffers, or the other form's flat one
-// (kGatherCap keys, from w.list on).
-struct GridLists {
-  WarpLists w;
-  unsigned long long more[kListCap];
+// Warps of a query CTA and keys of a warp: the flat buffer, whose first part is the
+// list form's three.  Two CTAs an SM: 16 warps with 512 keys each, but beside the
+// starts of 24^3 buckets 12 of those or, for short lists, 16 with 384 (one CTA
+// of 16 there: 8000 queries outside the palette's gamut against 62 000 entries, k
+// = 16, a whole call 1726 us, now 1100; 24 000 of k = 100 inside it 311 us, now 301,
+// and 329 with 384 keys).
+struct QueryShape {
+  int warps, keys;
 };
+__host__ __device__ constexpr QueryShape query_shape(int g, int k) {
+  return g < kMaxGridDim ? QueryShape{16, 4 * kListCap} : k <= 64 ? QueryShape{16, 3 * kListCap} : QueryShape{12, 4 * kListCap};
+}
+static_assert(sizeof(WarpLists) == 3 * kListCap * sizeof(unsigned long long), "the flat buffer's first part");
 
 struct Box {
   int x0, x1, y0, y1, z0, z1;  // inclusive bucket ranges
@@ -207,7 +212,7 @@ __device__ __forceinline__ void scan_box(const int* start, int g, const Box& o, 
 
 // ---- the select-then-sort query ------------------------------------------------------------
 // Most queries take this form: their candidate keys are gathered into the
-// warp's flat buffer (GridLists, kGatherCap keys), a distance that at least k of
+// warp's flat buffer (of kCap keys), a distance that at least k of
 // them lie within is found by bisection on the distance bits (a warp count per
 // step), the buffer is cut to the keys at or below it, and one bitonic sort of
 // what is left gives the k smallest keys -- instead of the top-k list's repeated
@@ -220,7 +225,6 @@ __device__ __forceinline__ void scan_box(const int* start, int g, const Box& o, 
 // entries 0.186 -> 0.110 ms, 470 000 against 10 000 1.88 -> 1.18; 24 000 against
 // 2600, 20 000 and 60 000 entries 0.143, 0.241 and 0.313 (with the new sort
 // alone) -> 0.101, 0.174 and 0.289.  640 keys: 10 000 entries 1.22.
-constexpr int kGatherCap = 4 * kListCap;
 
 // Appends the keys of box o (minus box in, when has_in) whose distance bits
 // are at most dthr to buf[n..); returns the new count (beyond cap: nothing
@@ -320,8 +324,9 @@ __device__ __forceinline__ uint32_t dist_bound(const unsigned long long* buf, in
   }
   return hi;
 }
+template <int kCap>
 __device__ __forceinline__ uint32_t kth_dist_bound(const unsigned long long* buf, int n, int k, int most, int lane) {
-  constexpr int kPer = kGatherCap / 32;
+  constexpr int kPer = kCap / 32;
   static_assert(kPer > 8, "the steps below");
   if (n <= 128) return dist_bound<4>(buf, n, k, most, lane);
   if (n <= 256) return dist_bound<8>(buf, n, k, most, lane);
@@ -356,21 +361,21 @@ __device__ __forceinline__ int count_box(const int* start, int g, const Box& b, 
   return (int)__reduce_add_sync(kFull, (unsigned)c);
 }
 
-__global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
+template <int kWarps, int kCap>
+__global__ void __launch_bounds__(kWarps * 32, 2) nearest_grid_kernel(
     const LabGrid* __restrict__ hdr, const float4* __restrict__ sorted, const int* __restrict__ start_g,
     const float4* __restrict__ queries, int nq, int k, int out_stride, uint32_t* __restrict__ out_idx,
     float* __restrict__ out_dist) {
   extern __shared__ __align__(16) uint8_t smem[];
-  GridLists* lists = reinterpret_cast<GridLists*>(smem);
-  int* start = reinterpret_cast<int*>(smem + kGridWarps * sizeof(GridLists));
+  int* start = reinterpret_cast<int*>(smem + sizeof(unsigned long long) * kWarps * kCap);
   const LabGrid H = *hdr;
   const int g = H.g, nb = g * g * g;
   for (int i = threadIdx.x; i <= nb; i += blockDim.x) start[i] = start_g[i];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WarpLists& W = lists[warp].w;
+  WarpLists& W = *reinterpret_cast<WarpLists*>(smem + sizeof(unsigned long long) * warp * kCap);
   const int target = min(H.p, kBoxFactor * k);
-  for (int qi = blockIdx.x * kGridWarps + warp; qi < nq; qi += gridDim.x * kGridWarps) {
+  for (int qi = blockIdx.x * kWarps + warp; qi < nq; qi += gridDim.x * kWarps) {
     const float4 q = queries[qi];
     int len = 0, nbuf = 0;
     unsigned long long thr = kMaxKey;
@@ -390,14 +395,14 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
       if (box_is_all(c, g)) cube_n = H.p;
     }
     // ---- select, then sort (the common form)
-    unsigned long long* fb = W.list;  // kGatherCap keys
+    unsigned long long* fb = W.list;  // kCap keys
     bool done = false;
-    if (cube_n <= kGatherCap) {
-      int m = gather_box(start, g, c, c, false, sorted, q, fb, 0, kGatherCap, 0xFFFFFFFFu, lane);
-      bool fits = m <= kGatherCap;
+    if (cube_n <= kCap) {
+      int m = gather_box(start, g, c, c, false, sorted, q, fb, 0, kCap, 0xFFFFFFFFu, lane);
+      bool fits = m <= kCap;
       if (fits && m > 0 && !box_is_all(c, g)) {
         // the cube holds >= min(P, k) entries: its k-th distance bounds the search
-        const uint32_t dk = kth_dist_bound(fb, m, min(k, m), k + k / 32, lane);
+        const uint32_t dk = kth_dist_bound<kCap>(fb, m, min(k, m), k + k / 32, lane);
         m = cut_keys(fb, m, dk, lane);
         if (m >= k && dk < kInfBits) {
           const float r = __fsqrt_rn(__uint_as_float(dk));
@@ -405,23 +410,23 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
           const Box o{grid_coord(__fsub_rn(q.x, R), H.lo[0], H.inv[0], g), grid_coord(__fadd_rn(q.x, R), H.lo[0], H.inv[0], g),
                       grid_coord(__fsub_rn(q.y, R), H.lo[1], H.inv[1], g), grid_coord(__fadd_rn(q.y, R), H.lo[1], H.inv[1], g),
                       grid_coord(__fsub_rn(q.z, R), H.lo[2], H.inv[2], g), grid_coord(__fadd_rn(q.z, R), H.lo[2], H.inv[2], g)};
-          m = gather_box(start, g, o, c, true, sorted, q, fb, m, kGatherCap, dk, lane);
+          m = gather_box(start, g, o, c, true, sorted, q, fb, m, kCap, dk, lane);
         } else {
           // fewer than k in the cube (palette below k), or fewer that are not NaN (those
           // lie in bucket 0, and sort behind every number): every entry counts
           const Box all{0, g - 1, 0, g - 1, 0, g - 1};
-          m = gather_box(start, g, all, c, true, sorted, q, fb, m, kGatherCap, 0xFFFFFFFFu, lane);
+          m = gather_box(start, g, all, c, true, sorted, q, fb, m, kCap, 0xFFFFFFFFu, lane);
         }
-        fits = m <= kGatherCap;
+        fits = m <= kCap;
       }
       if (fits && m > 0) {
         const int kk = min(k, m);
         int mp = 1;
         while (mp < kk) mp <<= 1;
-        const uint32_t d2 = kth_dist_bound(fb, m, kk, mp, lane);
+        const uint32_t d2 = kth_dist_bound<kCap>(fb, m, kk, mp, lane);
         m = cut_keys(fb, m, d2, lane);  // the k smallest keys and some more, at most mp but for ties
         while (mp < m) mp <<= 1;
-        if (mp <= kGatherCap) {
+        if (mp <= kCap) {
           for (int i = m + lane; i < mp; i += 32) fb[i] = kMaxKey;
           __syncwarp();
           warp_bitonic_sort(fb, mp, lane);
@@ -462,7 +467,9 @@ __global__ void __launch_bounds__(kGridThreads, 2) nearest_grid_kernel(
   }
 }
 
-size_t grid_query_smem(int g) { return kGridWarps * sizeof(GridLists) + sizeof(int) * ((size_t)g * g * g + 1); }
+size_t grid_query_smem(int g, QueryShape q) {
+  return sizeof(unsigned long long) * q.warps * q.keys + sizeof(int) * ((size_t)g * g * g + 1);
+}
 
 }  // namespace
 
@@ -490,8 +497,13 @@ int LabIndex::build(const float4* pal, int p, int method, int k, cudaStream_t s)
   if (configured_device != dev) {
     MG_CUDA(cudaFuncSetAttribute(lab_grid_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int) * kMaxGridDim * kMaxGridDim * kMaxGridDim)));
-    MG_CUDA(cudaFuncSetAttribute(nearest_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)grid_query_smem(kMaxGridDim)));
+    auto room = [](auto kernel, int g, int k) -> int {
+      MG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_query_smem(g, query_shape(g, k))));
+      return MG_OK;
+    };
+    MG_CHECK(room(nearest_grid_kernel<16, 4 * kListCap>, kMaxGridDim - 1, 1));
+    MG_CHECK(room(nearest_grid_kernel<16, 3 * kListCap>, kMaxGridDim, 1));
+    MG_CHECK(room(nearest_grid_kernel<12, 4 * kListCap>, kMaxGridDim, kListCap));
     configured_device = dev;
   }
   lab_grid_build_kernel<<<1, 1024, smem, s>>>(pal, p, g, hdr.as<LabGrid>(), sorted.as<float4>(), start.as<int>());
@@ -509,16 +521,21 @@ void LabIndex::release() {
 
 int launch_nearest_grid(const LabIndex& index, const float4* queries, int nq, int keff, int k, uint32_t* idx,
                         float* dist, cudaStream_t stream) {
-  const size_t smem = grid_query_smem(index.g);
+  const QueryShape shape = query_shape(index.g, keff);
+  const size_t smem = grid_query_smem(index.g, shape);
   int dev = 0, sms = 0, per_sm = 0;
   MG_CUDA(cudaGetDevice(&dev));
   MG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nearest_grid_kernel, kGridThreads, smem));
-  if (per_sm < 1) per_sm = 1;
-  const int groups = (nq + kGridWarps - 1) / kGridWarps;
-  const int grid = std::min(groups, sms * per_sm);
-  nearest_grid_kernel<<<grid, kGridThreads, smem, stream>>>(index.hdr.as<LabGrid>(), index.sorted.as<float4>(),
-                                                            index.start.as<int>(), queries, nq, keff, k, idx, dist);
+  auto go = [&](auto kernel) -> int {
+    MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * shape.warps, smem));
+    const int grid = std::min((nq + shape.warps - 1) / shape.warps, sms * std::max(per_sm, 1));
+    kernel<<<grid, 32 * shape.warps, smem, stream>>>(index.hdr.as<LabGrid>(), index.sorted.as<float4>(),
+                                                     index.start.as<int>(), queries, nq, keff, k, idx, dist);
+    return MG_OK;
+  };
+  MG_CHECK(shape.warps == 12 ? go(nearest_grid_kernel<12, 4 * kListCap>)
+           : shape.keys == 3 * kListCap ? go(nearest_grid_kernel<16, 3 * kListCap>)
+                                        : go(nearest_grid_kernel<16, 4 * kListCap>));
   g_launches += 1;
   MG_CUDA(cudaGetLastError());
   return MG_OK;
