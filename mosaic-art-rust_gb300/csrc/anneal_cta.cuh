@@ -42,8 +42,8 @@
 // levels on average), issue slots 39% used.  Before, a CTA of four warps drew,
 // evaluated, tested all pairs for conflicts and booked 32 (or 16) proposals in
 // turn, ~4 000 (2 550) cycles a round.  Measured, GB300, before -> now:
-// 64 chains x 100 000 iterations on 179 x 134 cells 6.32 -> 1.53 ms; 32 x 2000
-// on 80 x 60 0.203 -> 0.058 ms.  Windows of 32, eight lanes a proposal (16
+// 64 chains x 100 000 iterations on 179 x 134 cells 6.32 -> 1.49 ms; 32 x 2000
+// on 80 x 60 0.203 -> 0.060 ms.  Windows of 32, eight lanes a proposal (16
 // warps), and two proposals a group of eight lanes were measured too: 2.1, 1.55
 // and 2.0 ms on the first.
 #pragma once

@@ -43,11 +43,11 @@
 //    that are not there in time: ~500 cycles from trigger to list, ~1 000 when
 //    penalties decide.  Measured, GB300, before (records alone, no lists; 64
 //    scouts that read the counters through distributed shared memory) -> now:
-//    80 x 60 cells, 506 materials 0.551 -> 0.322 ms; 179 x 134, 5000 materials
-//    3.49 -> 1.74; 61 x 43, 112 materials, cap 2 0.518 -> 0.252; 64 mosaics of
+//    80 x 60 cells, 506 materials 0.551 -> 0.328 ms; 179 x 134, 5000 materials
+//    3.49 -> 1.77; 61 x 43, 112 materials, cap 2 0.518 -> 0.257; 64 mosaics of
 //    300 to 17 900 cells, 10 000 materials 4.6 -> 1.62; whole calls of 140 x 100
-//    cells, resets every few cells: 5 materials, cap 1 4.77 -> 4.41, 30 materials,
-//    cap 1 1.93 -> 1.84, 100 materials, cap 2 3.75 -> 1.32 (without the runs from
+//    cells, resets every few cells: 5 materials, cap 1 4.77 -> 4.30, 30 materials,
+//    cap 1 1.93 -> 1.77, 100 materials, cap 2 3.75 -> 1.28 (without the runs from
 //    records 6.4, 3.9 and 1.9).  Measured and not kept:
 //    blocks of 2 or 4 cells without branches (80 cycles a cell alone, but a list
 //    that is late costs a whole block), lists made 10, 14 or 20 cells ahead (late;
@@ -106,7 +106,7 @@ __host__ __device__ inline int scout_ahead(int gw, int p, uint32_t max_usage) {
 }
 // Lists of a cap-1 palette below this many materials would go unused: the cells
 // placed since a list was made have what it held (200 materials, cap 1: 2.68 ms
-// with them, 1.74 without; 1000 materials: 1.36 and 1.60).  Such a walk makes none
+// with them, 1.62 without; 1000 materials: 1.29 and 1.60).  Such a walk makes none
 // and goes by the records alone.
 constexpr int kCapOneLists = 512;
 __device__ __forceinline__ bool walks_by_lists(int p, uint32_t max_usage) {
@@ -1152,7 +1152,7 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   // before, or hold nothing.  Stops at a cell that its record does not settle
   // by a clear entry.  The word: position << 27 | not clear (or a counter that
   // does not fit) << 26 | counter << 16 | material.  Measured: 140 x 100 cells,
-  // 30 materials, cap 1: 3.89 -> 1.84 ms a call.  (Its result and what follows
+  // 30 materials, cap 1: 3.89 -> 1.77 ms a call.  (Its result and what follows
   // from it go through a shuffle: the compiler else takes the walker's loops for
   // divergent, 1.0 -> 1.4 ms for 5000 materials, which never come here.)
   int rec_ready = 0;  // the records of the cells from the walker's to before it are published
