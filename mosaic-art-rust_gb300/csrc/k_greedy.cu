@@ -1212,7 +1212,7 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
   while (c < n) {
     // the list of cell c, or, in a walk without lists, its record (bounded waits:
     // who makes them waits for nothing the walker has yet to do)
-    Entry e{0u, 0u};
+    Entry e = load_entry(c);
     if (lists) {
       // A cell passed by its list has been in its slot; a run from records leaves cells
       // behind whose lists may be late.  Until those are done, the walk stays
@@ -1224,8 +1224,8 @@ __global__ void __cluster_dims__(1 + kScoutCtas, 1, 1) __launch_bounds__(kThread
           if (gives_up(++polls)) break;
         if (aborted) break;
         behind = __shfl_sync(0xffffffffu, kNoneBehind, 0);
+        e = load_entry(c);  // (read before, it may be of two turns ago)
       }
-      e = load_entry(c);
       for (uint32_t polls = 0; !__all_sync(0xffffffffu, ((e.hi ^ list_tag(c, 0)) & kTagCell) == 0u);) {
         if (gives_up(++polls)) break;
         e = load_entry(c);
