@@ -43,8 +43,8 @@
 //    that are not there in time: ~500 cycles from trigger to list, ~1 000 when
 //    penalties decide.  Measured, GB300, before (records alone, no lists; 64
 //    scouts that read the counters through distributed shared memory) -> now:
-//    80 x 60 cells, 506 materials 0.551 -> 0.328 ms; 179 x 134, 5000 materials
-//    3.49 -> 1.77; 61 x 43, 112 materials, cap 2 0.518 -> 0.257; 64 mosaics of
+//    80 x 60 cells, 506 materials 0.551 -> 0.326 ms; 179 x 134, 5000 materials
+//    3.49 -> 1.75; 61 x 43, 112 materials, cap 2 0.518 -> 0.255; 64 mosaics of
 //    300 to 17 900 cells, 10 000 materials 4.6 -> 1.62; whole calls of 140 x 100
 //    cells, resets every few cells: 5 materials, cap 1 4.77 -> 4.30, 30 materials,
 //    cap 1 1.93 -> 1.77, 100 materials, cap 2 3.75 -> 1.28 (without the runs from
